@@ -335,14 +335,17 @@ CULIPX_API int culipx_factor_info(culipx_factor f, long long* info8)
     CULIPX_TRY(use_device(h));
     const Pattern& p = *f->pat;
     const int n = p.n, cm = p.num_blocks;
-    int u_nnz = 0, simple = 0;
+    long long u_nnz = 0;
+    int simple = 0;
     std::vector<int> flags(cm);
+    std::vector<int2> rng(n);
     CULIPX_CUDA(cudaStreamSynchronize(h->stream));
-    CULIPX_CUDA(cudaMemcpy(&u_nnz, f->u_off.as<int>() + n, sizeof(int), cudaMemcpyDeviceToHost));
+    CULIPX_CUDA(cudaMemcpy(rng.data(), f->u_rng.get(), n * sizeof(int2), cudaMemcpyDeviceToHost));
+    for (const int2& r : rng) u_nnz += r.y - r.x;
     CULIPX_CUDA(cudaMemcpy(&simple, f->scan_s.as<int>() + cm, sizeof(int), cudaMemcpyDeviceToHost));
     if (cm) CULIPX_CUDA(cudaMemcpy(flags.data(), f->rowflags.get(), cm * sizeof(int), cudaMemcpyDeviceToHost));
-    std::vector<int> extra(p.coarse_nnz);
-    if (p.coarse_nnz)
+    std::vector<int> extra(p.coarse_nnz, 0);
+    if (p.coarse_nnz && !f->two_level)
         CULIPX_CUDA(cudaMemcpy(extra.data(), f->got_extra.get(), p.coarse_nnz * sizeof(int), cudaMemcpyDeviceToHost));
     long long granted = 0;
     for (int v : extra) granted += (v > 0);

@@ -937,6 +937,34 @@ int run_levels(Factor* f, const void* d_vals, cudaStream_t s, int* launches)
 
 int build_sweeps(Factor* f, cudaStream_t stream, int* launches);  // solve.cu
 
+namespace {
+
+// The general path's block storage: with the factor for most patterns; for a
+// two-level one only once static pivots or a threshold call for it.
+int block_storage(Factor* f)
+{
+    const Pattern& p = *f->pat;
+    culipx_handle_t* h = p.handle;
+    const int cnz = p.coarse_nnz;
+    int st = CULIPX_OK;
+    auto al = [&](DeviceBuffer& buf, size_t bytes) {
+        if (st == CULIPX_OK && !buf.get()) st = buf.alloc(h, bytes ? bytes : 16);
+    };
+    al(f->val, f->val_cap * f->vbytes);
+    al(f->idx, f->val_cap * sizeof(int));
+    al(f->boff, cnz * sizeof(long long));
+    al(f->nnz, cnz * sizeof(int));
+    al(f->cap, cnz * sizeof(int));
+    al(f->got_extra, cnz * sizeof(int));
+    al(f->state, 16 * sizeof(long long));
+    al(f->deferred, (size_t)std::max(p.max_level_blocks, 1) * sizeof(int));
+    al(f->slowlist, (size_t)std::max(p.max_level_blocks, 1) * sizeof(int));
+    al(f->piv_off, p.num_blocks * sizeof(long long));
+    return st;
+}
+
+}  // namespace
+
 int factor_create(Pattern* p, Factor** out)
 {
     if (!p || !out) return fail(CULIPX_INVALID_ARG, "culipx_factor_create: null argument");
@@ -957,26 +985,24 @@ int factor_create(Pattern* p, Factor** out)
     auto al = [&](DeviceBuffer& buf, size_t bytes) {
         if (st == CULIPX_OK) st = buf.alloc(h, bytes ? bytes : 16);
     };
-    al(f->val, f->val_cap * f->vbytes);
-    al(f->idx, f->val_cap * sizeof(int));
-    al(f->boff, cnz * sizeof(long long));
-    al(f->nnz, cnz * sizeof(int));
-    al(f->cap, cnz * sizeof(int));
-    al(f->got_extra, cnz * sizeof(int));
+    if (!p->two_level) st = block_storage(f);
     al(f->tri, (3 * (size_t)n + 96) * f->vbytes);
     al(f->is_piv, (n + 32) * sizeof(int));
     al(f->perm, (n + 32) * sizeof(int));
     al(f->rowflags, cm * sizeof(int));
-    al(f->state, 16 * sizeof(long long));
-    al(f->deferred, (size_t)std::max(p->max_level_blocks, 1) * sizeof(int));
-    al(f->slowlist, (size_t)std::max(p->max_level_blocks, 1) * sizeof(int));
     al(f->u_off, (n + 1) * sizeof(int));
     al(f->ut_off, (n + 1) * sizeof(int));
+    al(f->u_rng, n * sizeof(int2));
+    al(f->ut_rng, n * sizeof(int2));
     al(f->u_col, off_slots * sizeof(int));
     al(f->ut_col, off_slots * sizeof(int));
     al(f->u_val, off_slots * f->vbytes);
     al(f->ut_val, off_slots * f->vbytes);
-    al(f->piv_off, cm * sizeof(long long));
+    if (p->two_level) {
+        al(f->kind, (cm + 15) / 16 * 16);
+        al(f->u_sub, (size_t)n * f->vbytes);
+        al(f->u_pair, 2 * (size_t)p->two_entries * f->vbytes);
+    }
     al(f->work, (size_t)n * f->vbytes);
     {
         // packed pivot tile triangles: h_I (h_I + 1) / 2 slots per block row,
@@ -1023,6 +1049,18 @@ int factor_compute(Factor* f, const void* d_vals, const int* h_is_piv, int pivot
             if (h_is_piv[i] != 0 && h_is_piv[i] != 1)
                 return fail(CULIPX_INVALID_ARG, "culipx_factor_compute: is_piv[%d] = %d is not 0/1", i, h_is_piv[i]);
     if (!f->capturing) CULIPX_CUDA(cudaEventRecord(h->ev_start, s));
+    // static pivots take given 2x2 pairs and thresholds need row norms: both
+    // stay on the general path, as do deeper patterns
+    f->two_level = p.two_level && pivot != CULIPX_PIV_STATIC && threshold == 0.0;
+    if (f->two_level) {
+        CULIPX_TRY(factor_two_level(f, d_vals, s, &launches));
+        if (!f->capturing) CULIPX_CUDA(cudaEventRecord(h->ev_stop, s));
+        f->last_launches = launches;
+        h->launches += launches;
+        f->computed = true;
+        return CULIPX_OK;
+    }
+    CULIPX_TRY(block_storage(f));
     CULIPX_CUDA(cudaMemsetAsync(f->val.get(), 0, p.val_slots * f->vbytes, s));
     CULIPX_CUDA(cudaMemcpyAsync(f->idx.get(), p.d_idx_init.get(), p.val_slots * sizeof(int),
                                 cudaMemcpyDeviceToDevice, s));
@@ -1113,11 +1151,101 @@ int factor_compute_graph(Factor* f, const void* d_vals, int pivot, double thresh
     CULIPX_CUDA(cudaEventRecord(h->ev_stop, s));
     f->pivot = pivot;
     f->threshold = threshold;
+    f->two_level = p.two_level && pivot != CULIPX_PIV_STATIC && threshold == 0.0;
     f->computed = true;
     f->last_launches = f->graph_launches;
     h->launches += f->graph_launches;
     return CULIPX_OK;
 }
+
+namespace {
+
+// The block form of a factor computed on fine rows: blocks in id order, each
+// level-0 block row's entries from its rows of U, the pivot tiles from their
+// packed triangles.
+int export_two_level(Factor* f, int* blk_nnz, long long* blk_off, int* idx, void* val, void* tri, int* is_piv,
+                     int* perm, int* got_extra, long long* total)
+{
+    Pattern& p = *f->pat;
+    cudaStream_t s = p.handle->stream;
+    const int cnz = p.coarse_nnz, n = p.n, cm = p.num_blocks;
+    const size_t vb = f->vbytes;
+    std::vector<int2> rng(n);
+    std::vector<int> flags(cm);
+    std::vector<long long> pko(cm + 1);
+    CULIPX_CUDA(cudaMemcpyAsync(rng.data(), f->u_rng.get(), n * sizeof(int2), cudaMemcpyDeviceToHost, s));
+    CULIPX_CUDA(cudaMemcpyAsync(flags.data(), f->rowflags.get(), cm * sizeof(int), cudaMemcpyDeviceToHost, s));
+    CULIPX_CUDA(cudaMemcpyAsync(pko.data(), f->pk_off.get(), (cm + 1) * sizeof(long long), cudaMemcpyDeviceToHost, s));
+    CULIPX_CUDA(cudaStreamSynchronize(s));
+    int slots = 0;
+    for (const int2& r : rng) slots = std::max(slots, r.y);
+    std::vector<int> col(slots);
+    std::vector<unsigned char> uv(slots * vb), pk(pko[cm] * vb);
+    if (slots) {
+        CULIPX_CUDA(cudaMemcpyAsync(col.data(), f->u_col.get(), slots * sizeof(int), cudaMemcpyDeviceToHost, s));
+        CULIPX_CUDA(cudaMemcpyAsync(uv.data(), f->u_val.get(), slots * vb, cudaMemcpyDeviceToHost, s));
+    }
+    std::vector<unsigned char> sub(n * vb);
+    CULIPX_CUDA(cudaMemcpyAsync(sub.data(), f->u_sub.get(), sub.size(), cudaMemcpyDeviceToHost, s));
+    CULIPX_CUDA(cudaMemcpyAsync(pk.data(), f->pk_row.get(), pk.size(), cudaMemcpyDeviceToHost, s));
+    CULIPX_CUDA(cudaStreamSynchronize(s));
+    unsigned char one[8];
+    const double one64 = 1.0;
+    const float one32 = 1.0f;
+    std::memcpy(one, vb == 8 ? (const void*)&one64 : (const void*)&one32, vb);
+    auto put = [&](long long at, const unsigned char* v) {
+        if (val) std::memcpy((unsigned char*)val + at * vb, v, vb);
+    };
+    long long o = 0;
+    std::vector<int> next(32);
+    for (int b = 0; b < cnz; ++b) {
+        const int I = p.blk_row[b], J = p.blk_col[b];
+        const int fr = p.bs[I], fc = p.bs[J];
+        const int r = p.bs[I + 1] - fr, c = p.bs[J + 1] - fc;
+        if (b == p.cs_off[I])
+            for (int i = 0; i < r; ++i) next[i] = rng[fr + i].x;
+        if (blk_off) blk_off[b] = o;
+        if (got_extra) got_extra[b] = 0;
+        const bool dense = p.fmt[b] == kDense;
+        if (dense) {
+            if (idx)
+                for (int e = 0; e < r * c; ++e) idx[o + e] = e;
+            if (val) std::memset((unsigned char*)val + o * vb, 0, (size_t)r * c * vb);
+        }
+        int cnt = 0;
+        if (I == J) {
+            for (int i = 0; i < r; ++i) {
+                if (i > 0 && (flags[I] & kRowHas2x2)) put(o + i * r + i - 1, &sub[(size_t)(fr + i) * vb]);
+                for (int j = i; j < r; ++j) {
+                    if (!(flags[I] & kRowIdentity))
+                        put(o + i * r + j, &pk[(pko[I] + i * r - i * (i - 1) / 2 + j - i) * vb]);
+                    else if (i == j)
+                        put(o + i * r + j, one);
+                }
+            }
+        } else {
+            for (int i = 0; i < r; ++i)
+                for (int& k = next[i]; k < rng[fr + i].y && col[k] < fc + c; ++k) {
+                    const int local = i * c + col[k] - fc;
+                    put(o + (dense ? local : cnt), &uv[(size_t)k * vb]);
+                    if (!dense) {
+                        if (idx) idx[o + cnt] = local;
+                        ++cnt;
+                    }
+                }
+        }
+        if (blk_nnz) blk_nnz[b] = cnt;
+        o += dense ? r * c : cnt;
+    }
+    if (blk_off) blk_off[cnz] = o;
+    if (total) *total = o;
+    if (tri) CULIPX_CUDA(cudaMemcpy(tri, f->tri.get(), 3 * (size_t)n * vb, cudaMemcpyDeviceToHost));
+    if (is_piv) CULIPX_CUDA(cudaMemcpy(is_piv, f->is_piv.get(), n * sizeof(int), cudaMemcpyDeviceToHost));
+    if (perm) CULIPX_CUDA(cudaMemcpy(perm, f->perm.get(), n * sizeof(int), cudaMemcpyDeviceToHost));
+    return CULIPX_OK;
+}
+
+}  // namespace
 
 int factor_export(Factor* f, int* blk_nnz, long long* blk_off, int* idx, void* val, void* tri, int* is_piv, int* perm,
                   int* got_extra, long long* total)
@@ -1125,6 +1253,7 @@ int factor_export(Factor* f, int* blk_nnz, long long* blk_off, int* idx, void* v
     if (!f->computed) return fail(CULIPX_INVALID_ARG, "culipx_factor_export: factor not computed");
     Pattern& p = *f->pat;
     cudaStream_t s = p.handle->stream;
+    if (f->two_level) return export_two_level(f, blk_nnz, blk_off, idx, val, tri, is_piv, perm, got_extra, total);
     const int cnz = p.coarse_nnz, n = p.n;
     std::vector<int> h_nnz(cnz), h_idx(f->val_cap), h_extra(cnz);
     std::vector<long long> h_boff(cnz);

@@ -53,9 +53,17 @@ struct Factor {
     DeviceBuffer norm_part;      // threshold > 0: row-norm partials
     DeviceBuffer row_norm;       // n values
 
-    // sweep structures (fine-row CSR of the strictly off-diagonal block part)
-    DeviceBuffer u_off, u_col, u_val;    // rows of U
+    // the last compute ran on K's fine rows (factor_two_level.cu): the block
+    // storage above was not written, the sweep structures below hold the factor
+    bool two_level = false;
+
+    // sweep structures (fine-row lists of the strictly off-diagonal block part)
+    DeviceBuffer u_off, u_col, u_val;    // rows of U (u_off: general path only)
     DeviceBuffer ut_off, ut_col, ut_val; // rows of U' (columns of U)
+    // factor_two_level.cu: a byte per level-1 block row; u and D u per entry;
+    // in block rows with 2x2 pivots the pivot tile's subdiagonal (export only)
+    DeviceBuffer kind, u_pair, u_sub;
+    DeviceBuffer u_rng, ut_rng;          // per fine row its entries' [first, end), as int2
     DeviceBuffer piv_off;                // per block row: value slot of its pivot tile
     // the persistent solver's copies: upper triangles of the non-identity
     // pivot tiles packed column by column (U sweep) and row by row (U'
@@ -101,6 +109,9 @@ int factor_compute(Factor* f, const void* d_vals, const int* h_is_piv, int pivot
 int factor_compute_graph(Factor* f, const void* d_vals, int pivot, double threshold);
 int factor_export(Factor* f, int* blk_nnz, long long* blk_off, int* idx, void* val, void* tri,
                   int* is_piv, int* perm, int* got_extra, long long* total);
+// factor.cu's launch sequence and build_sweeps in three launches, for patterns
+// with Pattern::two_level under BK / Rook pivoting without a drop threshold
+int factor_two_level(Factor* f, const void* d_vals, cudaStream_t stream, int* launches);
 int prec_apply(Factor* f, int stage, const void* d_b, void* d_x, cudaStream_t stream);
 
 }  // namespace culipx

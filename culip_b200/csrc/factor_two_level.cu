@@ -1,0 +1,554 @@
+// Numeric factorization on fine rows, for a two-level pattern whose level-0
+// block rows have diagonal pivot blocks (Pattern::two_level: a KKT system in
+// its natural order at fill level 0).
+//
+// There the factor has closed form up to the level-1 pivot tiles:
+//   level 0   D_g = K_gg (perturbed as d_ldlt_1x1_step does), U = I on the
+//             pivot blocks, U_gc = K_gc / D_g on the others;
+//   level 1   each block row's tile K_JJ - sum_g U_gJ' D_g U_gJ, factored with
+//             Bunch-Kaufman / Rook pivoting; no off-diagonal blocks.
+// The general path (factor.cu, solve.cu) stores U by blocks, updates a tile
+// block by block and then re-lays U out as fine rows.  Here K's rows are read
+// as they are and the fine rows are written at once, in three launches:
+//   k_two_rows    thread per level-0 row: D and the row of U
+//   k_two_tiles   warp per level-1 block row: the Schur update (a lane per
+//                 tile column), the tile's factorization, its packed triangles
+//                 and its rows of U'
+//   k_two_order   the rows of U into the order of the permuted columns; the
+//                 level-1 block rows split into simple ones and work items
+// Every value and every order of summation is the general path's: an update
+// block's contributions to a tile entry are summed in row order and then
+// subtracted, blocks in row order; entries of sparse blocks with |u| <= NZ_EPS
+// are dropped.
+//
+// Bound: the tiles' serial pivot steps and the dependent loads of the Schur
+// lists, not bandwidth.  Measured on the scale system (n = 200 000,
+// m = 100 000, 3125 tiles of 32, FP64): 147 us (rows 13, tiles 111, order 22)
+// against 960 us for the general path's 31 launches, 590 of them in the
+// tiles' block-by-block updates; N = 3000 with tiles of 4: 21 us against 130;
+// 256 systems of 2.0 M rows in FP32: 0.57 ms against 3.4.
+#include "factor.h"
+#include "kernels_common.cuh"
+#include "pivot_tile.cuh"
+
+#include <algorithm>
+
+namespace culipx {
+
+namespace {
+
+constexpr int kTileWarps = 4;   // level-1 block rows per CTA
+constexpr int kRowRegs = 8;     // entries of a row of U handled in registers
+
+template <class T>
+struct Pair {};
+template <>
+struct Pair<double> {
+    using type = double2;
+};
+template <>
+struct Pair<float> {
+    using type = float2;
+};
+
+template <class T>
+struct TwoArgs {
+    int n0;               // level-0 fine rows
+    int q1, nr1;          // first position of level 1 in lvl_rows, its block rows
+    int entries;          // of U, dropped ones included
+    int method;
+    double piv64;
+    const T* kval;
+    // the pattern's two-level form (pattern.h)
+    const int* kp;
+    const int* l0_rows;
+    const int* ucol;
+    const int2* low;
+    const int2* tail;
+    const int* tail_off;
+    const int* slot;
+    const int* l0_scan;
+    const int* lvl_rows;
+    const int* bs;
+    typename Pair<T>::type* up;  // per entry of U: u and D u, both 0 if dropped
+    T* u_sub;
+    T* tri;
+    T* dg;
+    int* is_piv;
+    int* perm;
+    int* rowflags;
+    int* u_col;
+    int* u_colp;
+    T* u_val;
+    int2* u_rng;
+    int* ut_col;
+    T* ut_val;
+    int2* ut_rng;
+    int* iperm;           // per level-1 fine row its place after the tile's swaps
+    const long long* pk_off;
+    T* pk_col;
+    T* pk_row;
+    unsigned* ndmask;
+    int* scan_s;
+    int* scan_c;
+    int* simple_rows;
+    int* cplx;
+    CItem* citem;
+    unsigned char* kind;  // per level-1 block row: its rows if simple, else 0
+};
+
+// a level-0 pivot from K's diagonal entry (0 if K stores none), perturbed as
+// d_ldlt_1x1_step (:556-560)
+template <class T>
+__device__ __forceinline__ T level0_pivot(const TwoArgs<T>& a, int tagged, int k0)
+{
+    T d = T(0);
+    if (!(tagged & two::kNoDiag)) d = __ldg(a.kval + k0);
+    if (fabs(d) < 1e-8) d = T(1e-6);
+    return d;
+}
+
+// Level-0 rows: D and the entries of U at their places of the pattern, each
+// with D u for the tiles' updates.  The left solve is k_offdiag_fast's Givens
+// form for a 1x1 pivot, its row constants taken once per row.
+template <class T>
+__global__ void __launch_bounds__(256) k_two_rows(TwoArgs<T> a)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= a.n0) return;
+    const int tagged = __ldg(a.l0_rows + i);
+    const int g = tagged & two::kRowMask;
+    const int k0 = __ldg(a.kp + g), k1 = __ldg(a.kp + g + 1);
+    const int o0 = __ldg(a.slot + g);
+    const T d11 = level0_pivot(a, tagged, k0);
+    const T d22 = (tagged & two::kNextInBlock) ? level0_pivot(a, __ldg(a.l0_rows + i + 1), k1) : T(0);
+    const T d12 = T(0);
+    const T gr = sqrt(fma_rn(d11, d11, d12 * d12));
+    const T gc = d11 / gr, gs = d12 / gr;
+    const T td11 = fma_rn(gc, d11, gs * d12);
+    const T td12 = fma_rn(gc, d12, gs * d22);
+    const int kb = (tagged & two::kNoDiag) ? k0 : k0 + 1;
+    for (int k = kb; k < k1; k += kRowRegs) {
+        T v[kRowRegs];
+#pragma unroll
+        for (int j = 0; j < kRowRegs; ++j) v[j] = (k + j < k1) ? __ldg(a.kval + k + j) : T(0);
+#pragma unroll
+        for (int j = 0; j < kRowRegs; ++j) {
+            if (k + j >= k1) break;
+            const int o = o0 + (k + j - kb);
+            T u = fma_rn(gc, v[j], gs * T(0));
+            u = fma_rn(-td12, T(0), u) / td11;
+            // sparse blocks drop |u| <= NZ_EPS, dense ones keep every non-zero
+            if (!(fabs(u) > T(kNzEps)) && !((tagged & two::kRowDense) && __ldg(a.ucol + o) < 0)) u = T(0);
+            typename Pair<T>::type e;
+            e.x = u;
+            e.y = d11 * u;
+            if (u == T(0)) e.y = T(0);
+            a.up[o] = e;
+        }
+    }
+    a.ut_rng[g] = make_int2(0, 0);
+    a.dg[g] = d11;
+    a.tri[3 * (size_t)g] = T(0);
+    a.tri[3 * (size_t)g + 1] = d11;
+    a.tri[3 * (size_t)g + 2] = T(0);
+    a.perm[g] = g;
+    a.is_piv[g] = 1;
+    a.simple_rows[i] = g;
+}
+
+// One entry of a level-1 row with what its update needs: its own u and D u,
+// and the two entries before it in the level-0 row (ahead of use).
+template <class T>
+struct LowEntry {
+    int g, before, slot;
+    T u, du;
+    int c1, c2;
+    T du1, du2;
+};
+
+template <class T>
+__device__ __forceinline__ void load_low(const TwoArgs<T>& a, int2 w, LowEntry<T>& e)
+{
+    e.g = w.x;
+    e.before = (int)((unsigned)w.y >> two::kBeforeShift);
+    e.slot = w.y & two::kSlotMask;
+    const auto q = a.up[e.slot];
+    e.u = q.x;
+    e.du = q.y;
+    e.c1 = e.c2 = 0;
+    e.du1 = e.du2 = T(0);
+    if (e.before > 0) {
+        e.c1 = __ldg(a.ucol + e.slot - 1);
+        e.du1 = a.up[e.slot - 1].y;
+    }
+    if (e.before > 1) {
+        e.c2 = __ldg(a.ucol + e.slot - 2);
+        e.du2 = a.up[e.slot - 2].y;
+    }
+}
+
+// One level-1 block row per warp.  Lane b owns column b of the tile's upper
+// triangle (T_ab at tile[a][b], a <= b) and keeps the running sums of the
+// current update block in the mirrored places (tile[b][a], a < b; the
+// diagonal's in a register), so the update needs no synchronisation and the
+// tile is all the shared memory a warp holds.  The lane walks K's row fr + b:
+// each entry's column g is a level-0 row whose entries inside the tile up to
+// column b are the update's factors; they stand next to each other in U, so
+// the pattern holds the entry's place and the count before it, and the loads
+// of the next two entries are in flight while one is used.
+template <class T>
+__global__ void __launch_bounds__(32 * kTileWarps) k_two_tiles(TwoArgs<T> a)
+{
+    __shared__ T tiles[kTileWarps][kTileElems];
+    __shared__ int perm_s[kTileWarps][32];
+    __shared__ int piv_s[kTileWarps][32];
+    const int warp = threadIdx.x >> 5;
+    const int t = blockIdx.x * kTileWarps + warp;
+    if (t >= a.nr1) return;
+    const int b = lane_id();
+    T* tile = tiles[warp];
+    const int I = __ldg(a.lvl_rows + a.q1 + t);
+    const int fr = __ldg(a.bs + I), h = __ldg(a.bs + I + 1) - fr;
+    const int me = fr + b;
+    int k0 = 0, k1 = 0;
+    if (b < h) {
+        k0 = __ldg(a.slot + me);
+        // the rows' lists follow each other in level order, the last one ends with U
+        if (b + 1 < h) k1 = __ldg(a.slot + me + 1);
+        else k1 = (t + 1 < a.nr1) ? __ldg(a.slot + __ldg(a.bs + __ldg(a.lvl_rows + a.q1 + t + 1))) : a.entries;
+    }
+    for (int e = b; e < kTileElems; e += 32) tile[e] = T(0);
+    __syncwarp();
+    for (int k = __ldg(a.tail_off + t) + b; k < __ldg(a.tail_off + t + 1); k += 32) {
+        const int2 e = __ldg(a.tail + k);
+        tile[(e.y >> 5) * kTileStride + (e.y & 31)] = __ldg(a.kval + e.x);
+    }
+    __syncwarp();
+
+    int ut = k0;
+    T pdiag = T(0);
+    unsigned touched = 0;
+    T* const col = tile + b;
+    T* const sum = tile + b * kTileStride;
+    auto subtract = [&]() {
+        while (touched) {
+            const int r = __ffs(touched) - 1;
+            touched &= touched - 1;
+            if (r == b) {
+                col[r * kTileStride] -= pdiag;
+                pdiag = T(0);
+            } else {
+                col[r * kTileStride] -= sum[r];
+                sum[r] = T(0);
+            }
+        }
+    };
+    LowEntry<T> cur, nxt;
+    int2 ahead = make_int2(0, 0);
+    if (k0 < k1) load_low(a, __ldg(a.low + k0), cur);
+    if (k0 + 1 < k1) ahead = __ldg(a.low + k0 + 1);
+    for (int k = k0; k < k1; ++k) {
+        if (k + 1 < k1) load_low(a, ahead, nxt);
+        if (k + 2 < k1) ahead = __ldg(a.low + k + 2);
+        if (cur.g >= 0) subtract();  // another update block begins
+        if (cur.u != T(0)) {         // not dropped
+            a.ut_col[ut] = cur.g & two::kColMask;
+            a.ut_val[ut] = cur.u;
+            ++ut;
+            auto add = [&](int r, T du) {
+                if (du == T(0)) return;
+                touched |= 1u << r;
+                sum[r] = fma_rn(cur.u, du, sum[r]);
+            };
+            for (int q = cur.before; q > 2; --q)
+                add((__ldg(a.ucol + cur.slot - q) & two::kColMask) - fr, a.up[cur.slot - q].y);
+            if (cur.before > 1) add((cur.c2 & two::kColMask) - fr, cur.du2);
+            if (cur.before > 0) add((cur.c1 & two::kColMask) - fr, cur.du1);
+            if (cur.du != T(0)) {
+                touched |= 1u << b;
+                pdiag = fma_rn(cur.u, cur.du, pdiag);
+            }
+        }
+        cur = nxt;
+    }
+    subtract();
+    __syncwarp();
+
+    int* perm = perm_s[warp];
+    int* piv = piv_s[warp];
+    T* D = a.tri + 3 * (size_t)fr;
+    perm[b] = b;
+    piv[b] = 1;
+    __syncwarp();
+    bool diag = true;
+    for (int r = 0; r < h; ++r) diag &= b <= r || b >= h || tile[r * kTileStride + b] == T(0);
+    if (__all_sync(0xffffffffu, diag)) {
+        // 1x1 pivots without swaps (k_pivot_blocks' short cut)
+        if (b < h) {
+            T d = tile[b * kTileStride + b];
+            if (fabs(d) < 1e-8) d = T(1e-6);
+            tile[b * kTileStride + b] = T(1);
+            D[3 * b] = T(0);
+            D[3 * b + 1] = d;
+            D[3 * b + 2] = T(0);
+        }
+        __syncwarp();
+    } else {
+        factorize_tile(tile, h, piv, D, perm, a.method, a.piv64);
+    }
+    __syncwarp();
+
+    bool ident = true;
+    if (b < h)
+        for (int r = 0; r <= b; ++r) ident &= tile[r * kTileStride + b] == (r == b ? T(1) : T(0));
+    ident = __all_sync(0xffffffffu, ident);
+    const bool two = __any_sync(0xffffffffu, b < h && (D[3 * b + 2] != T(0) || D[3 * b] != T(0)));
+    const bool pid = __all_sync(0xffffffffu, b >= h || perm[b] == b);
+    const unsigned nd = __ballot_sync(0xffffffffu, b < h && tile[b * kTileStride + b] != T(1));
+    if (b == 0) {
+        a.rowflags[I] = (ident ? kRowIdentity : 0) | (two ? kRowHas2x2 : 0) | (pid ? kRowPermIdentity : 0);
+        a.ndmask[I] = nd;
+        a.kind[t] = (ident && pid && !two) ? (unsigned char)h : 0;
+    }
+    const int from = (b < h) ? perm[b] : b;  // the column now at place b
+    const int s0 = shfl(k0, from), s1 = shfl(ut, from);
+    if (b < h) {
+        a.dg[me] = D[3 * b + 1];
+        a.is_piv[me] = piv[b];
+        a.perm[me] = fr + from;
+        a.iperm[fr + from] = me;
+        a.ut_rng[me] = make_int2(s0, s1);
+        a.u_rng[me] = make_int2(0, 0);
+    }
+    // a 2x2 pivot's rounding residue left of its second row's diagonal, for the export
+    if (two && b < h) a.u_sub[me] = b > 0 ? tile[b * kTileStride + b - 1] : T(0);
+    if (!ident) {
+        T* pc = a.pk_col + __ldg(a.pk_off + I);
+        T* pr = a.pk_row + __ldg(a.pk_off + I);
+        for (int r = 0; r < h; ++r)
+            if (b >= r && b < h) {
+                const T v = tile[r * kTileStride + b];
+                pc[b * (b + 1) / 2 + r] = v;
+                pr[r * h - r * (r - 1) / 2 + b - r] = v;
+            }
+    }
+}
+
+// The first split CTAs: the lists of solve.cu's k_split_count / k_split_fill, kOrderT
+// level-1 block rows each, their prefix summed from one byte per earlier tile
+// (the rows of a simple one, 0 for a work item; level 0 is all simple).  The
+// others: a thread per level-0 row sorts its entries by their columns' places
+// after the tiles' swaps (swaps stay inside a block, so rows keep their block
+// order) and maps them back through the permutation.
+constexpr int kOrderT = 256;
+
+template <class T>
+__device__ void split_rows(const TwoArgs<T>& a, int q0)
+{
+    __shared__ int sum_s[kOrderT / 32], sum_c[kOrderT / 32];
+    const int tid = threadIdx.x, lane = lane_id(), w = tid >> 5;
+    int s = 0, c = 0;  // simple rows and work items of this thread's share of the tiles before q0
+    const uint4* kinds = reinterpret_cast<const uint4*>(a.kind);
+    for (int i = tid; i < q0 / 16; i += kOrderT) {
+        const uint4 v = __ldg(kinds + i);
+        const unsigned words[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            s += (int)__dp4a(words[j], 0x01010101u, 0u);
+            c += __popc(__vcmpeq4(words[j], 0u)) / 8;
+        }
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        s += __shfl_xor_sync(0xffffffffu, s, o);
+        c += __shfl_xor_sync(0xffffffffu, c, o);
+    }
+    if (lane == 0) {
+        sum_s[w] = s;
+        sum_c[w] = c;
+    }
+    __syncthreads();
+    s = a.n0;
+    c = 0;
+    for (int k = 0; k < kOrderT / 32; ++k) {
+        s += sum_s[k];
+        c += sum_c[k];
+    }
+    __syncthreads();
+    const int t = q0 + tid, q = a.q1 + t;
+    const bool in = t < a.nr1;
+    const int rows = in ? a.kind[t] : 0;
+    const int item = in && rows == 0;
+    int is = rows, ic = item;
+    for (int o = 1; o < 32; o <<= 1) {
+        const int x = __shfl_up_sync(0xffffffffu, is, o), y = __shfl_up_sync(0xffffffffu, ic, o);
+        if (lane >= o) {
+            is += x;
+            ic += y;
+        }
+    }
+    if (lane == 31) {
+        sum_s[w] = is;
+        sum_c[w] = ic;
+    }
+    __syncthreads();
+    s += is - rows;
+    c += ic - item;
+    for (int k = 0; k < w; ++k) {
+        s += sum_s[k];
+        c += sum_c[k];
+    }
+    if (!in) return;
+    a.scan_s[q] = s;
+    a.scan_c[q] = c;
+    const int I = __ldg(a.lvl_rows + q);
+    const int fr = __ldg(a.bs + I);
+    for (int r = 0; r < rows; ++r) a.simple_rows[s + r] = fr + r;
+    if (item) {
+        CItem it;
+        it.I = I;
+        it.fr = fr;
+        it.h = __ldg(a.bs + I + 1) - fr;
+        it.flags = a.rowflags[I];
+        it.pk_off = __ldg(a.pk_off + I);
+        it.nd = a.ndmask[I];
+        it.pad = 0;
+        a.cplx[c] = I;
+        a.citem[c] = it;
+    }
+    if (t == a.nr1 - 1) {
+        a.scan_s[q + 1] = s + rows;
+        a.scan_c[q + 1] = c + item;
+    }
+}
+
+template <class T>
+__global__ void __launch_bounds__(kOrderT) k_two_order(TwoArgs<T> a, int splits)
+{
+    if ((int)blockIdx.x < splits) {
+        split_rows(a, blockIdx.x * kOrderT);
+        return;
+    }
+    const int i = ((int)blockIdx.x - splits) * kOrderT + threadIdx.x;
+    if (i < a.q1) {  // the level-0 block rows' entries of the lists
+        a.scan_s[i] = __ldg(a.l0_scan + i);
+        a.scan_c[i] = 0;
+        a.rowflags[__ldg(a.lvl_rows + i)] = kRowIdentity | kRowPermIdentity | kRowNoUpdates;
+    }
+    if (i >= a.n0) return;
+    const int tagged = __ldg(a.l0_rows + i);
+    const int g = tagged & two::kRowMask;
+    const int o0 = __ldg(a.slot + g);
+    const int len = __ldg(a.kp + g + 1) - __ldg(a.kp + g) - ((tagged & two::kNoDiag) ? 0 : 1);
+    if (len <= kRowRegs) {
+        int c[kRowRegs], nc[kRowRegs];
+        T v[kRowRegs];
+#pragma unroll
+        for (int j = 0; j < kRowRegs; ++j) {
+            c[j] = (j < len) ? __ldg(a.ucol + o0 + j) & two::kColMask : -1;
+            v[j] = (j < len) ? a.up[o0 + j].x : T(0);
+        }
+        int kept = 0;
+#pragma unroll
+        for (int j = 0; j < kRowRegs; ++j) {
+            const bool keep = v[j] != T(0);
+            nc[j] = keep ? __ldg(a.iperm + c[j]) : two::kColMask;
+            kept += keep;
+        }
+#pragma unroll
+        for (int j = 0; j < kRowRegs; ++j) {
+            int rank = 0;
+#pragma unroll
+            for (int k = 0; k < kRowRegs; ++k)
+                if (k != j) rank += nc[k] < nc[j];
+            if (v[j] != T(0)) {
+                a.u_colp[o0 + rank] = c[j];
+                a.u_col[o0 + rank] = nc[j];
+                a.u_val[o0 + rank] = v[j];
+            }
+        }
+        a.u_rng[g] = make_int2(o0, o0 + kept);
+        return;
+    }
+    int o = o0;
+    for (int j = 0; j < len; ++j) {  // insertion: an entry moves within its block's few
+        const T v = a.up[o0 + j].x;
+        if (v == T(0)) continue;
+        const int c = __ldg(a.ucol + o0 + j) & two::kColMask, nc = __ldg(a.iperm + c);
+        int k = o++;
+        for (; k > o0 && a.u_col[k - 1] > nc; --k) {
+            a.u_col[k] = a.u_col[k - 1];
+            a.u_colp[k] = a.u_colp[k - 1];
+            a.u_val[k] = a.u_val[k - 1];
+        }
+        a.u_col[k] = nc;
+        a.u_colp[k] = c;
+        a.u_val[k] = v;
+    }
+    a.u_rng[g] = make_int2(o0, o);
+}
+
+template <class T>
+int run(Factor* f, const void* d_vals, cudaStream_t s, int* launches)
+{
+    const Pattern& p = *f->pat;
+    TwoArgs<T> a;
+    a.n0 = p.l0_count;
+    a.q1 = p.lvl_off[1];
+    a.nr1 = p.lvl_off[2] - p.lvl_off[1];
+    a.method = f->pivot;
+    a.piv64 = f->pivot_fp64;
+    a.entries = p.two_entries;
+    a.kval = static_cast<const T*>(d_vals);
+    a.kp = p.two_kp;
+    a.l0_rows = p.two_l0_rows;
+    a.ucol = p.two_ucol;
+    a.low = p.two_low;
+    a.tail = p.two_tail;
+    a.tail_off = p.two_tail_off;
+    a.up = f->u_pair.as<typename Pair<T>::type>();
+    a.slot = p.two_slot;
+    a.l0_scan = p.two_l0_scan;
+    a.lvl_rows = p.d_lvl_rows.as<int>();
+    a.bs = p.d_bs.as<int>();
+    a.u_sub = f->u_sub.as<T>();
+    a.tri = f->tri.as<T>();
+    a.dg = f->dg.as<T>();
+    a.is_piv = f->is_piv.as<int>();
+    a.perm = f->perm.as<int>();
+    a.rowflags = f->rowflags.as<int>();
+    a.u_col = f->u_col.as<int>();
+    a.u_colp = f->u_colp.as<int>();
+    a.u_val = f->u_val.as<T>();
+    a.u_rng = f->u_rng.as<int2>();
+    a.ut_col = f->ut_col.as<int>();
+    a.ut_val = f->ut_val.as<T>();
+    a.ut_rng = f->ut_rng.as<int2>();
+    a.iperm = f->u_off.as<int>();
+    a.pk_off = f->pk_off.as<long long>();
+    a.pk_col = f->pk_col.as<T>();
+    a.pk_row = f->pk_row.as<T>();
+    a.ndmask = f->ndmask.as<unsigned>();
+    a.scan_s = f->scan_s.as<int>();
+    a.scan_c = f->scan_c.as<int>();
+    a.simple_rows = f->simple_rows.as<int>();
+    a.cplx = f->cplx.as<int>();
+    a.citem = f->citem.as<CItem>();
+    a.kind = f->kind.as<unsigned char>();
+    k_two_rows<T><<<(a.n0 + 255) / 256, 256, 0, s>>>(a);
+    k_two_tiles<T><<<(a.nr1 + kTileWarps - 1) / kTileWarps, 32 * kTileWarps, 0, s>>>(a);
+    const int splits = (a.nr1 + kOrderT - 1) / kOrderT;
+    k_two_order<T><<<(a.n0 + kOrderT - 1) / kOrderT + splits, kOrderT, 0, s>>>(a, splits);
+    *launches += 3;
+    return launch_check("two-level factorization");
+}
+
+}  // namespace
+
+int factor_two_level(Factor* f, const void* d_vals, cudaStream_t s, int* launches)
+{
+    if (f->precision == CULIPX_F64) return run<double>(f, d_vals, s, launches);
+    return run<float>(f, d_vals, s, launches);
+}
+
+}  // namespace culipx

@@ -19,6 +19,19 @@ struct BlockDesc {
     int cap;      // sparse: capacity in entries (max_nnz); dense: r*c
 };
 
+// Packing of the two-level form's arrays (Pattern::d_l0_rows, d_ucol, d_low).
+namespace two {
+constexpr int kNextInBlock = 1 << 30;         // l0_rows: the next fine row is in the same block
+constexpr int kRowDense = 1 << 29;            // l0_rows: the row has entries in dense blocks
+constexpr int kNoDiag = (int)0x80000000u;     // l0_rows: K stores no diagonal entry for the row
+constexpr int kRowMask = kRowDense - 1;
+constexpr int kDense = (int)0x80000000u;      // ucol: the entry is in a dense block
+constexpr int kColMask = 0x7fffffff;
+constexpr int kSameBlock = (int)0x80000000u;  // low.x: same block row as the entry before it
+constexpr int kBeforeShift = 27;              // low.y: entries of the same row and tile before it, over
+constexpr int kSlotMask = (1 << 27) - 1;      //        its slot in U
+}  // namespace two
+
 struct Pattern {
     culipx_handle_t* handle = nullptr;
     // the creator's reference plus one per factor / batch made from it through
@@ -45,6 +58,13 @@ struct Pattern {
     // between two rows of the same level-0 block row): a level-0 row's K row
     // then reads only itself and rows of later levels
     bool l0_diagonal = false;
+    // two levels whose level-0 block rows have diagonal pivot blocks, rows of
+    // moderate length (a KKT system in its natural order at fill level 0): the
+    // factor runs on K's fine rows (factor_two_level.cu).  The device arrays
+    // below exist for such patterns only.
+    bool two_level = false;
+    int l0_count = 0;             // fine rows of level 0
+    int two_entries = 0;          // entries of U
     std::vector<int> lb_off, lb;  // factor order per level: pivots, then off-diagonal (CSR order)
     // per row position t of lvl_rows: index of the row's first off-diagonal
     // block inside its level's off-diagonal list
@@ -65,6 +85,15 @@ struct Pattern {
     DeviceBuffer d_row_offdiag_start, d_lvl_off;
     DeviceBuffer d_cs_off, d_desc, d_bs, d_csc_off, d_csc_blk, d_lb, d_lvl_rows, d_a_dst, d_idx_init,
         d_nnz_init, d_fmt, d_maxnnz, d_row_block;
+    // two_level, parts of d_two: K's row offsets; the level-0 fine rows; the
+    // columns of U's entries, row after row; the entries of U', level-1 row
+    // after level-1 row; K's own entries of the level-1 pivot tiles with their
+    // offsets per tile; per fine row its first entry in U (level 0) or U'
+    // (level 1); per level-0 position of lvl_rows the fine rows before it
+    DeviceBuffer d_two;
+    const int *two_kp = nullptr, *two_l0_rows = nullptr, *two_ucol = nullptr, *two_tail_off = nullptr,
+              *two_slot = nullptr, *two_l0_scan = nullptr;
+    const int2 *two_low = nullptr, *two_tail = nullptr;
     long long device_bytes = 0;
 };
 

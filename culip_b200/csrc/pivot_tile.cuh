@@ -82,29 +82,39 @@ __device__ __forceinline__ void pivot_swap(T* Tt, int* perm, int p1, int p2, int
     __syncwarp();
 }
 
-// argmax of v over lanes, ties to the lowest index (value, index) = (v, i).
-// A NaN score counts as 0 (no candidate): with NaNs the comparisons are no
-// total order and the lanes' butterflies would end at different results.
+// The largest of the lanes' non-negative values, as bits: their order is that
+// of the values.  Two (FP32: one) warp reductions instead of five rounds of
+// shuffles.
+__device__ __forceinline__ float max_bits(float v)
+{
+    return __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(v)));
+}
+
+__device__ __forceinline__ double max_bits(double v)
+{
+    const unsigned hi = (unsigned)__double2hiint(v), lo = (unsigned)__double2loint(v);
+    const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
+    const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
+    return __hiloint2double((int)mh, (int)ml);
+}
+
+// argmax of the lanes' v >= 0, ties to the lowest index (value, index) =
+// (v, i), with i increasing over the lanes that hold a positive v.  A NaN
+// score counts as 0 (no candidate), so every lane ends at the same result.
 template <class T>
 __device__ __forceinline__ void warp_argmax(T& v, int& i)
 {
     if (v != v) v = T(0);
-    for (int o = 16; o > 0; o >>= 1) {
-        const T ov = __shfl_xor_sync(0xffffffffu, v, o);
-        const int oi = __shfl_xor_sync(0xffffffffu, i, o);
-        if (ov > v || (ov == v && oi < i)) { v = ov; i = oi; }
-    }
+    const T m = max_bits(v);
+    if (m > T(0)) i = shfl(i, __ffs(__ballot_sync(0xffffffffu, v == m)) - 1);
+    else i = __reduce_min_sync(0xffffffffu, i);
+    v = m;
 }
 
 template <class T>
 __device__ __forceinline__ T warp_max(T v)
 {
-    if (v != v) v = T(0);  // as in warp_argmax: every lane ends at the same value
-    for (int o = 16; o > 0; o >>= 1) {
-        const T ov = __shfl_xor_sync(0xffffffffu, v, o);
-        v = (ov > v) ? ov : v;
-    }
-    return v;
+    return max_bits(v != v ? T(0) : v);
 }
 
 template <class T>
@@ -173,6 +183,7 @@ __device__ __forceinline__ void step_1x1(T* Tt, T* D, int row, int len)
     __syncwarp();
     Tt[row * kTileStride + l] = u;
     const T ru = u * d11;
+#pragma unroll 4
     for (int i = row + 1; i < len; ++i) {
         const T lv = shfl(ru, i);
         if (l < len) Tt[i * kTileStride + l] = fma_rn(-lv, u, Tt[i * kTileStride + l]);

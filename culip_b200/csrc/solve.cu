@@ -480,19 +480,23 @@ __global__ void k_split_fill(int cm, const int* __restrict__ lvl_rows, const int
 }
 
 // U's column indices mapped through the pivot permutation (the persistent
-// solver gathers the finished U-sweep values from P t directly), and the
-// diagonal of D
+// solver gathers the finished U-sweep values from P t directly), the
+// diagonal of D, and each fine row's range of entries
 template <class T>
 __global__ void k_sweep_extras(const int* __restrict__ u_off, const int* __restrict__ u_col,
                                const int* __restrict__ perm, int* __restrict__ u_colp, int n,
-                               const T* __restrict__ tri, T* __restrict__ dg)
+                               const T* __restrict__ tri, T* __restrict__ dg, const int* __restrict__ ut_off,
+                               int2* __restrict__ u_rng, int2* __restrict__ ut_rng)
 {
     const long long nu = u_off[n];
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < nu; k += stride)
         u_colp[k] = perm[u_col[k]];
-    for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < n; g += stride)
+    for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < n; g += stride) {
         dg[g] = tri[3 * g + 1];
+        u_rng[g] = make_int2(u_off[g], u_off[g + 1]);
+        ut_rng[g] = make_int2(ut_off[g], ut_off[g + 1]);
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -511,7 +515,7 @@ __global__ void k_sweep_extras(const int* __restrict__ u_off, const int* __restr
 template <class T, bool UPPER>
 __global__ void __launch_bounds__(32 * kSweepWarps)
     k_sweep_level(const int* __restrict__ rows, int nrows, const int* __restrict__ bs,
-                  const int* __restrict__ off, const int* __restrict__ col, const T* __restrict__ vals,
+                  const int2* __restrict__ rng, const int* __restrict__ col, const T* __restrict__ vals,
                   const long long* __restrict__ pk_off, const int* __restrict__ rowflags,
                   const T* __restrict__ pk, const int* __restrict__ perm, const T* src, T* x)
 {
@@ -533,8 +537,9 @@ __global__ void __launch_bounds__(32 * kSweepWarps)
         // the row's terms in batches of 8: index and value loads, then the
         // gathers, then the fmas in column order
         constexpr int B = 8;
-        const int e1 = off[g + 1];
-        for (int k = off[g]; k < e1; k += B) {
+        const int2 kr = rng[g];
+        const int e1 = kr.y;
+        for (int k = kr.x; k < e1; k += B) {
             int c[B];
             T v[B], xv[B];
 #pragma unroll
@@ -585,12 +590,13 @@ __global__ void __launch_bounds__(32 * kSweepWarps)
 // and 2635-2674): x_out_I = U_II^-1 (b_I - U_I* x_in) for U (UPPER) or U'
 template <class T, bool UPPER>
 __global__ void __launch_bounds__(32 * kSweepWarps)
-    k_sweep_jacobi(int cm, const int* __restrict__ bs, const int* __restrict__ off, const int* __restrict__ col,
-                   const T* __restrict__ vals, const long long* __restrict__ piv_off,
-                   const int* __restrict__ rowflags, const T* __restrict__ fval, const T* __restrict__ b,
+    k_sweep_jacobi(int cm, const int* __restrict__ bs, const int2* __restrict__ rng, const int* __restrict__ col,
+                   const T* __restrict__ vals, const long long* __restrict__ pk_off,
+                   const int* __restrict__ rowflags, const T* __restrict__ pk_row, const T* __restrict__ b,
                    const T* __restrict__ x_in, T* __restrict__ x_out)
 {
-    __shared__ T tiles[kSweepWarps][kTileElems];
+    constexpr int kTri = 32 * 33 / 2;
+    __shared__ T tiles[kSweepWarps][kTri];
     const int warp = threadIdx.x >> 5;
     const int I = blockIdx.x * kSweepWarps + warp;
     if (I >= cm) return;
@@ -599,26 +605,27 @@ __global__ void __launch_bounds__(32 * kSweepWarps)
     T acc = T(0);
     if (lane < h) {
         acc = b[fr + lane];
-        const int e1 = off[fr + lane + 1];
-        for (int k = off[fr + lane]; k < e1; ++k) acc = fma_rn(-vals[k], x_in[col[k]], acc);
+        const int2 kr = rng[fr + lane];
+        for (int k = kr.x; k < kr.y; ++k) acc = fma_rn(-vals[k], x_in[col[k]], acc);
     }
     if (!(rowflags[I] & kRowIdentity)) {
         T* tile = tiles[warp];
-        const T* P = fval + piv_off[I];
-        if (lane < h)
-            for (int i = 0; i < h; ++i) tile[i * kTileStride + lane] = P[i * h + lane];
+        const T* P = pk_row + pk_off[I];
+        for (int e = lane; e < h * (h + 1) / 2; e += 32) tile[e] = P[e];
         __syncwarp();
+        // row r of the triangle at r h - r (r - 1) / 2: columns r .. h - 1
+        auto at = [&](int r, int c) { return tile[r * h - r * (r - 1) / 2 + c - r]; };
         if (UPPER) {
             for (int c = h - 1; c >= 0; --c) {
-                if (lane == c) acc = acc / tile[c * kTileStride + c];
+                if (lane == c) acc = acc / at(c, c);
                 const T xc = shfl(acc, c);
-                if (lane < c) acc = fma_rn(-tile[lane * kTileStride + c], xc, acc);
+                if (lane < c) acc = fma_rn(-at(lane, c), xc, acc);
             }
         } else {
             for (int r = 0; r < h; ++r) {
-                if (lane == r) acc = acc / tile[r * kTileStride + r];
+                if (lane == r) acc = acc / at(r, r);
                 const T xr = shfl(acc, r);
-                if (lane > r && lane < h) acc = fma_rn(-tile[r * kTileStride + lane], xr, acc);
+                if (lane > r && lane < h) acc = fma_rn(-at(r, lane), xr, acc);
             }
         }
     }
@@ -711,7 +718,8 @@ int build_sweeps_t(Factor* f, cudaStream_t s, int* launches)
         cm, a.bs, f->piv_off.as<long long>(), f->rowflags.as<int>(), val, f->pk_off.as<long long>(),
         f->pk_col.as<T>(), f->pk_row.as<T>(), f->ndmask.as<unsigned>());
     k_sweep_extras<T><<<148 * 4, 256, 0, s>>>(u_off, f->u_col.as<int>(), f->perm.as<int>(), f->u_colp.as<int>(), n,
-                                              f->tri.as<T>(), f->dg.as<T>());
+                                              f->tri.as<T>(), f->dg.as<T>(), ut_off, f->u_rng.as<int2>(),
+                                              f->ut_rng.as<int2>());
     const int* lvl_rows = p.d_lvl_rows.as<int>();
     const int* rowflags = f->rowflags.as<int>();
     k_split_count<<<std::min(cm / 256 + 1, 148 * 4), 256, 0, s>>>(cm, lvl_rows, a.bs, rowflags, f->scan_s.as<int>(),
@@ -739,7 +747,6 @@ int apply_t(Factor* f, int stage, const void* d_b, void* d_x, cudaStream_t s)
         k_solve_D<T><<<grid_n, 256, 0, s>>>(f->tri.as<T>(), f->is_piv.as<int>(), b, x, n, f->pivot_fp64);
         return launch_check("k_solve_D");
     }
-    const T* fval = f->val.as<T>();
     if (f->solve_algorithm == CULIPX_SOLVE_JACOBI) {
         // x = 0, then `sweeps` block-Jacobi sweeps on the right-hand side rhs
         if (!f->jac_a.get()) CULIPX_TRY(f->jac_a.alloc(p.handle, (size_t)n * sizeof(T) + 16));
@@ -756,12 +763,12 @@ int apply_t(Factor* f, int stage, const void* d_b, void* d_x, cudaStream_t s)
         for (int sw = 0; sw < f->jacobi_sweeps; ++sw) {
             if (left)
                 k_sweep_jacobi<T, false><<<grid, 32 * kSweepWarps, 0, s>>>(
-                    cm, p.d_bs.as<int>(), f->ut_off.as<int>(), f->ut_col.as<int>(), f->ut_val.as<T>(),
-                    f->piv_off.as<long long>(), f->rowflags.as<int>(), fval, rhs, xa, xb);
+                    cm, p.d_bs.as<int>(), f->ut_rng.as<int2>(), f->ut_col.as<int>(), f->ut_val.as<T>(),
+                    f->pk_off.as<long long>(), f->rowflags.as<int>(), f->pk_row.as<T>(), rhs, xa, xb);
             else
                 k_sweep_jacobi<T, true><<<grid, 32 * kSweepWarps, 0, s>>>(
-                    cm, p.d_bs.as<int>(), f->u_off.as<int>(), f->u_col.as<int>(), f->u_val.as<T>(),
-                    f->piv_off.as<long long>(), f->rowflags.as<int>(), fval, rhs, xa, xb);
+                    cm, p.d_bs.as<int>(), f->u_rng.as<int2>(), f->u_col.as<int>(), f->u_val.as<T>(),
+                    f->pk_off.as<long long>(), f->rowflags.as<int>(), f->pk_row.as<T>(), rhs, xa, xb);
             std::swap(xa, xb);
         }
         if (left) CULIPX_CUDA(cudaMemcpyAsync(x, xa, n * sizeof(T), cudaMemcpyDeviceToDevice, s));
@@ -780,7 +787,7 @@ int apply_t(Factor* f, int stage, const void* d_b, void* d_x, cudaStream_t s)
         for (int L = 0; L < p.num_levels; ++L) {
             const int nr = p.lvl_off[L + 1] - p.lvl_off[L];
             k_sweep_level<T, false><<<(nr + kSweepWarps - 1) / kSweepWarps, 32 * kSweepWarps, 0, s>>>(
-                p.d_lvl_rows.as<int>() + p.lvl_off[L], nr, p.d_bs.as<int>(), f->ut_off.as<int>(),
+                p.d_lvl_rows.as<int>() + p.lvl_off[L], nr, p.d_bs.as<int>(), f->ut_rng.as<int2>(),
                 f->ut_col.as<int>(), f->ut_val.as<T>(), f->pk_off.as<long long>(), f->rowflags.as<int>(),
                 f->pk_row.as<T>(), f->perm.as<int>(), src, x);
         }
@@ -790,7 +797,7 @@ int apply_t(Factor* f, int stage, const void* d_b, void* d_x, cudaStream_t s)
     for (int L = p.num_levels - 1; L >= 0; --L) {
         const int nr = p.lvl_off[L + 1] - p.lvl_off[L];
         k_sweep_level<T, true><<<(nr + kSweepWarps - 1) / kSweepWarps, 32 * kSweepWarps, 0, s>>>(
-            p.d_lvl_rows.as<int>() + p.lvl_off[L], nr, p.d_bs.as<int>(), f->u_off.as<int>(), f->u_colp.as<int>(),
+            p.d_lvl_rows.as<int>() + p.lvl_off[L], nr, p.d_bs.as<int>(), f->u_rng.as<int2>(), f->u_colp.as<int>(),
             f->u_val.as<T>(), f->pk_off.as<long long>(), f->rowflags.as<int>(), f->pk_col.as<T>(),
             f->perm.as<int>(), b, x);
     }

@@ -55,10 +55,10 @@ PArgs<TF> make_args(Csr* A, Factor* M, double* base, double* partials, const dou
     a.lvl_off = p.d_lvl_off.as<int>();
     a.lvl_rows = p.d_lvl_rows.as<int>();
     a.bs = p.d_bs.as<int>();
-    a.u_off = M->u_off.as<int>();
+    a.u_rng = M->u_rng.as<int2>();
     a.u_colp = M->u_colp.as<int>();
     a.u_val = M->u_val.as<TF>();
-    a.ut_off = M->ut_off.as<int>();
+    a.ut_rng = M->ut_rng.as<int2>();
     a.ut_col = M->ut_col.as<int>();
     a.ut_val = M->ut_val.as<TF>();
     a.rowflags = M->rowflags.as<int>();
@@ -507,6 +507,7 @@ int batch_factor_solve_graph(Batch* bt, Csr* A, Factor* M, const void* d_vals, i
     h->launches += bt->graph_launches;
     M->pivot = pivot;
     M->threshold = threshold;
+    M->two_level = M->pat->two_level && pivot != CULIPX_PIV_STATIC && threshold == 0.0;
     M->computed = true;
     return batch_results(bt, max_it, h_res, h_its, h_status);
 }

@@ -98,10 +98,10 @@ struct PArgs {
     const int* lvl_off;
     const int* lvl_rows;
     const int* bs;
-    const int* u_off;
+    const int2* u_rng;         // per fine row: its entries' [first, end)
     const int* u_colp;         // U columns mapped through P
     const TF* u_val;
-    const int* ut_off;
+    const int2* ut_rng;
     const int* ut_col;
     const TF* ut_val;
     const int* rowflags;
@@ -568,10 +568,11 @@ __device__ void res_load(const PArgs<TF>& a, ResSlot<TF>& rs, int t, bool has)
     if (lane < h) {
         const int g = fr + lane;
         rs.q[lane] = (m.flags & kRowPermIdentity) ? g : __ldg(a.perm + g);
-        rs.u0[lane] = __ldg(a.u_off + g);
-        rs.u1[lane] = __ldg(a.u_off + g + 1);
-        rs.ut0[lane] = __ldg(a.ut_off + g);
-        rs.ut1[lane] = __ldg(a.ut_off + g + 1);
+        const int2 ur = __ldg(a.u_rng + g), utr = __ldg(a.ut_rng + g);
+        rs.u0[lane] = ur.x;
+        rs.u1[lane] = ur.y;
+        rs.ut0[lane] = utr.x;
+        rs.ut1[lane] = utr.y;
         rs.d[lane] = (m.flags & kRowHas2x2) ? 1.0 : (double)__ldg(a.dg + g);
     }
     if (!(m.flags & kRowIdentity))
@@ -619,7 +620,8 @@ __device__ __forceinline__ void u_item(const PArgs<TF>& a, const ItemMeta& m, co
         TF acc[NR];
 #pragma unroll
         for (int r = 0; r < NR; ++r) acc[r] = (TF)d[r];
-        row_sub<TF, NR>(acc, __ldg(a.u_off + fr + lane), __ldg(a.u_off + fr + lane + 1), a.u_colp, a.u_val, out);
+        const int2 kr = __ldg(a.u_rng + fr + lane);
+        row_sub<TF, NR>(acc, kr.x, kr.y, a.u_colp, a.u_val, out);
 #pragma unroll
         for (int r = 0; r < NR; ++r) t[r] = (double)acc[r];
     }
@@ -666,8 +668,8 @@ __device__ __forceinline__ void ut_item(const PArgs<TF>& a, const ItemMeta& m, c
         TF acc[NR];
 #pragma unroll
         for (int r = 0; r < NR; ++r) acc[r] = (TF)y[r];
-        row_sub<TF, NR, SCG>(acc, __ldg(a.ut_off + fr + lane), __ldg(a.ut_off + fr + lane + 1), a.ut_col, a.ut_val,
-                             dst, sc);
+        const int2 kr = __ldg(a.ut_rng + fr + lane);
+        row_sub<TF, NR, SCG>(acc, kr.x, kr.y, a.ut_col, a.ut_val, dst, sc);
 #pragma unroll
         for (int r = 0; r < NR; ++r) t[r] = (double)acc[r];
     }
@@ -1184,7 +1186,8 @@ __device__ void sqmr_body(const PArgs<TF>& a, Ctx& ctx, const SysView& sv, Scal 
                         level_wait(it);
                         ready = true;
                     }
-                    row_sub<TF, NR>(acc, __ldg(a.u_off + g), __ldg(a.u_off + g + 1), a.u_colp, a.u_val, a.ev);
+                    const int2 kr = __ldg(a.u_rng + g);
+                    row_sub<TF, NR>(acc, kr.x, kr.y, a.u_colp, a.u_val, a.ev);
 #pragma unroll
                     for (int j = 0; j < NR; ++j) a.ev[(size_t)g * NR + j] = (double)acc[j];
                     if (fz) {
@@ -1354,11 +1357,11 @@ __device__ void sqmr_body(const PArgs<TF>& a, Ctx& ctx, const SysView& sv, Scal 
                         scv[j] = cf.sc[j];
                         acc[j] = (TF)(y[j] * scv[j]);
                     }
+                    const int2 kr = __ldg(a.ut_rng + g);
                     if (fused)  // level 1: its U' rows gather the unscaled level-0 Av
-                        row_sub<TF, NR, true>(acc, __ldg(a.ut_off + g), __ldg(a.ut_off + g + 1), a.ut_col, a.ut_val,
-                                              a.Av, scv);
+                        row_sub<TF, NR, true>(acc, kr.x, kr.y, a.ut_col, a.ut_val, a.Av, scv);
                     else
-                        row_sub<TF, NR>(acc, __ldg(a.ut_off + g), __ldg(a.ut_off + g + 1), a.ut_col, a.ut_val, a.Av);
+                        row_sub<TF, NR>(acc, kr.x, kr.y, a.ut_col, a.ut_val, a.Av);
                     double av[NR];
 #pragma unroll
                     for (int j = 0; j < NR; ++j) {
