@@ -3,6 +3,7 @@
 
 #include "device.h"
 #include "spmv.h"
+#include "sqmr_lockstep.h"
 
 #include <vector>
 
@@ -20,6 +21,7 @@ struct Sqmr {
     DeviceBuffer vecs, partials, scal;
     DeviceBuffer ref_r, ref_d, ref_part;  // iterative refinement: residual, correction, norm partials
     DeviceBuffer ref_best;                // its best iterate so far
+    DeviceBuffer lock;                    // batched solve on the whole grid: sums, scalars, coefficients
     DeviceBuffer many;                    // sqmr_solve_many: vectors, argument blocks, counter
     void* host_flags = nullptr;  // pinned
     ~Sqmr()
@@ -39,6 +41,7 @@ struct Batch {
     std::vector<int> row_off;                 // num + 1
     DeviceBuffer d_row_off, d_qb, d_qe;       // num + 1, num x nl, num x nl
     DeviceBuffer d_out, d_next;               // num x 8 results, system counter
+    LockPlan lock;                            // two-level patterns: the work units of sqmr_lockstep.cu
     // batch_factor_solve_graph: the factorization and the batched solve as one
     // CUDA graph, its own workspace (the graph holds its addresses), and what
     // the graph was captured for

@@ -3,8 +3,8 @@
 namespace culipx {
 
 namespace persistent {
-CULIPX_SQMR_BATCHED(, float)
-CULIPX_SQMR_MANY(, float, false)
+CULIPX_SQMR_BATCHED(float)
+CULIPX_SQMR_MANY(float, false)
 }  // namespace persistent
 
 }  // namespace culipx

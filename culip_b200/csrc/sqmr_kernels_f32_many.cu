@@ -3,7 +3,7 @@
 namespace culipx {
 
 namespace persistent {
-CULIPX_SQMR_MANY(, float, true)
+CULIPX_SQMR_MANY(float, true)
 }  // namespace persistent
 
 }  // namespace culipx

@@ -3,8 +3,8 @@
 namespace culipx {
 
 namespace persistent {
-CULIPX_SQMR_BATCHED(, double)
-CULIPX_SQMR_MANY(, double, false)
+CULIPX_SQMR_BATCHED(double)
+CULIPX_SQMR_MANY(double, false)
 }  // namespace persistent
 
 }  // namespace culipx

@@ -3,7 +3,7 @@
 namespace culipx {
 
 namespace persistent {
-CULIPX_SQMR_MANY(, double, true)
+CULIPX_SQMR_MANY(double, true)
 }  // namespace persistent
 
 }  // namespace culipx

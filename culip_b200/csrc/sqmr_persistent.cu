@@ -11,21 +11,6 @@ namespace culipx {
 
 using namespace persistent;
 
-namespace persistent {
-CULIPX_SQMR_PERSISTENT(extern, double, 1)
-CULIPX_SQMR_PERSISTENT(extern, double, 2)
-CULIPX_SQMR_PERSISTENT(extern, double, 4)
-CULIPX_SQMR_PERSISTENT(extern, float, 1)
-CULIPX_SQMR_PERSISTENT(extern, float, 2)
-CULIPX_SQMR_PERSISTENT(extern, float, 4)
-CULIPX_SQMR_BATCHED(extern, double)
-CULIPX_SQMR_BATCHED(extern, float)
-CULIPX_SQMR_MANY(extern, double, false)
-CULIPX_SQMR_MANY(extern, double, true)
-CULIPX_SQMR_MANY(extern, float, false)
-CULIPX_SQMR_MANY(extern, float, true)
-}  // namespace persistent
-
 namespace {
 
 // kernel arguments over a work area of kVecs n nr doubles + 8 nr (vectors, then out)
@@ -97,7 +82,7 @@ int ctas_per_sm()
 template <class TF, int NR>
 const void* persistent_kernel()
 {
-    return ctas_per_sm() == 1 ? (const void*)k_sqmr_persistent<TF, 1, NR> : (const void*)k_sqmr_persistent<TF, 2, NR>;
+    return ctas_per_sm() == 1 ? persistent_fn<TF, 1, NR>() : persistent_fn<TF, 2, NR>();
 }
 
 // resident CTAs for the cooperative launch
@@ -300,6 +285,32 @@ int sqmr_solve_multi_async(culipx_handle_t* h, Csr* A, Factor* M, int nrhs, cons
 // block-diagonal union pattern.
 namespace {
 
+// The whole-grid solve (a two-level factor, A on its pattern).
+template <class TF>
+int launch_lockstep(Batch* bt, const PArgs<TF>& a, Sqmr* w)
+{
+    culipx_handle_t* h = bt->h;
+    const size_t need = lockstep_bytes(a.n, bt->num);
+    if (w->lock.bytes() < need) CULIPX_TRY(w->lock.alloc(h, need));
+    static DeviceGridCache grid_cache;  // one per factor precision
+    int G = 0;
+    CULIPX_TRY(cached_grid(
+        grid_cache,
+        [](int dev, int* g) {
+            int per_sm = 0, sms = 0;
+            CULIPX_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+            CULIPX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, lockstep_kernel<TF>(), kT, 0));
+            if (per_sm < 1) return fail(CULIPX_NOT_SUPPORTED, "lockstep SQMR kernel does not fit on an SM");
+            *g = sms * std::min(per_sm, kCtasPerSm);
+            return (int)CULIPX_OK;
+        },
+        &G));
+    CULIPX_TRY(lockstep_launch<TF>(a, bt->lock, bt->num, bt->d_row_off.as<int>(), bt->d_qb.as<int>(),
+                                   bt->d_qe.as<int>(), w->lock.get(), bt->d_out.as<double>(), G, h->stream));
+    h->launches += 1;
+    return CULIPX_OK;
+}
+
 template <class TF>
 int launch_batched(Batch* bt, Csr* A, Factor* M, const double* b, double* x, double tol, int max_it, Sqmr* w)
 {
@@ -314,7 +325,7 @@ int launch_batched(Batch* bt, Csr* A, Factor* M, const double* b, double* x, dou
         [](int dev, int* g) {
             int per_sm = 0, sms = 0;
             CULIPX_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-            CULIPX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sqmr_batched<TF>, kT, 0));
+            CULIPX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batched_fn<TF>(), kT, 0));
             if (per_sm < 1) return fail(CULIPX_NOT_SUPPORTED, "batched SQMR kernel does not fit on an SM");
             *g = sms * std::min(per_sm, kCtasPerSm);
             return (int)CULIPX_OK;
@@ -330,10 +341,50 @@ int launch_batched(Batch* bt, Csr* A, Factor* M, const double* b, double* x, dou
     ba.next = bt->d_next.as<int>();
     CULIPX_CUDA(cudaMemsetAsync(a.v[0], 0, (size_t)kVecs * n * sizeof(double), s));
     CULIPX_CUDA(cudaMemsetAsync(x, 0, (size_t)n * sizeof(double), s));
+    // static pivots or a threshold leave a factor whose level 0 is not known to be simple
+    if (bt->lock.use && M->two_level && a.fuse_l0) return launch_lockstep<TF>(bt, a, w);
     CULIPX_CUDA(cudaMemsetAsync(ba.next, 0, sizeof(int), s));
-    k_sqmr_batched<TF><<<std::min(G, bt->num), kT, 0, s>>>(a, ba);
+    void* args[] = {&a, &ba};
+    CULIPX_CUDA(cudaLaunchKernel(batched_fn<TF>(), dim3(std::min(G, bt->num)), dim3(kT), args, 0, s));
     h->launches += 1;
-    return launch_check("k_sqmr_batched");
+    return CULIPX_OK;
+}
+
+}  // namespace
+
+namespace {
+
+// The work units of the whole-grid solve, where it gains.  One CTA per system
+// lasts as long as its largest system: measured 25 + 17.5 per 1000 rows us an
+// iteration (FP32 and FP64 alike, the device not full); the whole grid takes
+// 60 for its synchronisations, 0.15 per 1000 rows of all systems and 2.4 per
+// 1000 rows of the largest for its sums.  256 systems of 750 to 30 000 rows:
+// 0.84 ms against 0.46; one system of 30 000 rows: 0.55 against 0.09; 296
+// systems of 4500 rows: 0.20 against 0.29, which keep a CTA each.  Both kernels
+// give the same bits, so the choice does not show in the results.
+int lockstep_plan(culipx_handle_t* h, const Pattern& p, int num, const int* row_off, const std::vector<int>& qb,
+                  const std::vector<int>& qe, LockPlan& plan)
+{
+    int largest = 0;
+    for (int s = 0; s < num; ++s) largest = std::max(largest, row_off[s + 1] - row_off[s]);
+    plan.use = 25.0 + 17.5e-3 * largest > 60.0 + 0.15e-3 * p.n + 2.4e-3 * largest;
+    if (!plan.use) return CULIPX_OK;
+    std::vector<int4> chunk, tile;
+    int pos = 0;  // level 0's fine rows in level-list order
+    for (int s = 0; s < num; ++s) {
+        int rows = 0;
+        for (int q = qb[2 * s]; q < qe[2 * s]; ++q) rows += p.bs[p.lvl_rows[q] + 1] - p.bs[p.lvl_rows[q]];
+        for (int r = 0; r < rows; r += 32) chunk.push_back(make_int4(pos + r, std::min(32, rows - r), s, 0));
+        pos += rows;
+        for (int q = qb[2 * s + 1]; q < qe[2 * s + 1]; ++q) {
+            const int I = p.lvl_rows[q];
+            tile.push_back(make_int4(I, p.bs[I], p.bs[I + 1] - p.bs[I], s));
+        }
+    }
+    plan.chunks = (int)chunk.size();
+    plan.tiles = (int)tile.size();
+    chunk.insert(chunk.end(), tile.begin(), tile.end());
+    return plan.units.upload(h, chunk.data(), chunk.size() * sizeof(int4));
 }
 
 }  // namespace
@@ -382,6 +433,7 @@ int batch_create(culipx_handle_t* h, const Pattern* p, int num, const int* h_row
     if (st == CULIPX_OK) st = bt->d_qe.upload(h, qe.data(), qe.size() * sizeof(int));
     if (st == CULIPX_OK) st = bt->d_out.alloc(h, (size_t)num * 8 * sizeof(double));
     if (st == CULIPX_OK) st = bt->d_next.alloc(h, sizeof(int));
+    if (st == CULIPX_OK && p->two_level) st = lockstep_plan(h, *p, num, h_row_off, qb, qe, bt->lock);
     if (st != CULIPX_OK) {
         delete bt;
         return st;
@@ -599,12 +651,16 @@ int launch_many_prec(culipx_handle_t* h, const std::vector<int>& ks, const int* 
         };
     };
     int G = 0;
-    if (multi) CULIPX_TRY(cached_grid(grid_caches[1], many_grid((const void*)k_sqmr_many<TF, true>), &G));
-    else CULIPX_TRY(cached_grid(grid_caches[0], many_grid((const void*)k_sqmr_many<TF, false>), &G));
-    if (multi) k_sqmr_many<TF, true><<<std::min(G, num), kT, 0, s>>>(d_args, d_nr, num, d_next);
-    else k_sqmr_many<TF, false><<<std::min(G, num), kT, 0, s>>>(d_args, d_nr, num, d_next);
+    if (multi) CULIPX_TRY(cached_grid(grid_caches[1], many_grid(many_fn<TF, true>()), &G));
+    else CULIPX_TRY(cached_grid(grid_caches[0], many_grid(many_fn<TF, false>()), &G));
+    const PArgs<TF>* arg_sys = d_args;
+    const int* arg_nr = d_nr;
+    int arg_num = num;
+    int* arg_next = d_next;
+    void* kargs[] = {&arg_sys, &arg_nr, &arg_num, &arg_next};
+    CULIPX_CUDA(cudaLaunchKernel(multi ? many_fn<TF, true>() : many_fn<TF, false>(), dim3(std::min(G, num)), dim3(kT),
+                                 kargs, 0, s));
     h->launches += 1;
-    CULIPX_TRY(launch_check("k_sqmr_many"));
     for (int i = 0; i < num; ++i)
         CULIPX_CUDA(cudaMemcpyAsync(out_host + 8 * slot[ks[i]], args[i].out, (size_t)8 * nrs[i] * sizeof(double),
                                     cudaMemcpyDeviceToHost, s));

@@ -766,6 +766,69 @@ inline __device__ void sym_ortho(double a, double b, double& c, double& s, doubl
     }
 }
 
+// The recurrence after a U sweep: rr = ||v+||^2 (unscaled) gives delta and the
+// rotation of step k (k0, k1, km1: the places of k, k + 1, k - 1).
+inline __device__ void scal_after_u(Scal& Q, double rr, int k0, int k1, int km1)
+{
+    const double alpha = Q.alpha_next;
+    Q.alpha = alpha;
+    const double bk = Q.beta[k0];
+    const double dl = sqrt(rr);
+    Q.delta[k1] = dl;
+    Q.inv_delta = 1.0 / dl;
+    const double nA = sqrt(fma_rn(dl, dl, fma_rn(alpha, alpha, bk * bk)));
+    Q.norm_A = fmax(Q.norm_A, nA);
+    Q.epsilon = Q.s[km1] * bk;
+    const double beta_rot = (-Q.c[km1]) * bk;
+    Q.beta_rr = fma_rn(Q.c[k0], beta_rot, Q.s[k0] * alpha);
+    const double alpha_rot = fma_rn(Q.s[k0], beta_rot, (-Q.c[k0]) * alpha);
+    double c, s, rho;
+    sym_ortho(alpha_rot, dl, c, s, rho);
+    Q.c[k1] = c;
+    Q.s[k1] = s;
+    Q.rho = rho;
+    Q.inv_rho = 1.0 / rho;
+    Q.tau = c * Q.gamma;
+    Q.gamma = s * Q.gamma;
+}
+
+// The recurrence after a U' sweep: vda = v_k' D^-1 Av, wda = v+' D^-1 Av, wdw
+// = v+' D^-1 v+, xx = ||x||^2; beta, the next alpha and the lagged tests.
+inline __device__ void scal_after_ut(Scal& Q, double vda, double wda, double wdw, double xx, int it, int k1,
+                                     double tol, int max_it)
+{
+    const double bt = vda / Q.vdv;
+    Q.beta[k1] = bt;
+    Q.inv_beta = 1.0 / bt;
+    Q.eta = (Q.delta[k1] / bt) * Q.eta;
+    Q.alpha_next = wda / wdw;
+    Q.vdv = wdw;
+    Q.norm_x = sqrt(xx);
+    Q.test0 |= (fabs(Q.delta[k1]) <= tol);
+    Q.test1 |= (Q.gamma / fma_rn(Q.norm_A, Q.norm_x, Q.norm_pb) <= tol);
+    bool stop = false;
+    if (it > 0 && (it % 4) == 0) {
+        if (Q.snap0 || Q.snap1) {
+            stop = true;
+            Q.iters = it;
+        }
+    } else if (((it + 1) % 4) == 0) {
+        Q.snap0 = Q.test0;
+        Q.snap1 = Q.test1;
+    }
+    if (!isfinite(Q.inv_beta) || !isfinite(Q.inv_rho) || !isfinite(Q.eta) || !isfinite(Q.inv_delta) ||
+        !isfinite(Q.alpha)) {
+        Q.breakdown = 1;
+        stop = true;
+        Q.iters = it;
+    }
+    if (!stop && it + 1 >= max_it) Q.iters = max_it;
+    if (stop) {
+        Q.done = 1;
+        Q.stop_it = it;
+    }
+}
+
 // Fixed-order sum over one CTA: thread 0 gets the totals (same protocol as
 // grid_reduce).
 template <int NV>
@@ -1215,27 +1278,7 @@ __device__ void sqmr_body(const PArgs<TF>& a, Ctx& ctx, const SysView& sv, Scal 
             if (tid == 0)
                 for (int j = 0; j < NR; ++j) {
                     if (S[j].done) continue;
-                    Scal& Q = S[j];
-                    const double alpha = Q.alpha_next;
-                    Q.alpha = alpha;
-                    const double bk = Q.beta[k0];
-                    const double dl = sqrt(r[j]);
-                    Q.delta[k1] = dl;
-                    Q.inv_delta = 1.0 / dl;
-                    const double nA = sqrt(fma_rn(dl, dl, fma_rn(alpha, alpha, bk * bk)));
-                    Q.norm_A = fmax(Q.norm_A, nA);
-                    Q.epsilon = Q.s[km1] * bk;
-                    const double beta_rot = (-Q.c[km1]) * bk;
-                    Q.beta_rr = fma_rn(Q.c[k0], beta_rot, Q.s[k0] * alpha);
-                    const double alpha_rot = fma_rn(Q.s[k0], beta_rot, (-Q.c[k0]) * alpha);
-                    double c, s, rr;
-                    sym_ortho(alpha_rot, dl, c, s, rr);
-                    Q.c[k1] = c;
-                    Q.s[k1] = s;
-                    Q.rho = rr;
-                    Q.inv_rho = 1.0 / rr;
-                    Q.tau = c * Q.gamma;
-                    Q.gamma = s * Q.gamma;
+                    scal_after_u(S[j], r[j], k0, k1, km1);
                 }
             if (tid == 0)
                 for (int j = 0; j < NR; ++j) {
@@ -1400,38 +1443,8 @@ __device__ void sqmr_body(const PArgs<TF>& a, Ctx& ctx, const SysView& sv, Scal 
             ctx.template reduce<4 * NR>(r, sh);
             if (tid == 0)
                 for (int j = 0; j < NR; ++j) {
-                    Scal& Q = S[j];
-                    if (Q.done) continue;
-                    const double bt = r[j] / Q.vdv;
-                    Q.beta[k1] = bt;
-                    Q.inv_beta = 1.0 / bt;
-                    Q.eta = (Q.delta[k1] / bt) * Q.eta;
-                    Q.alpha_next = r[NR + j] / r[2 * NR + j];
-                    Q.vdv = r[2 * NR + j];
-                    Q.norm_x = sqrt(r[3 * NR + j]);
-                    Q.test0 |= (fabs(Q.delta[k1]) <= a.tol);
-                    Q.test1 |= (Q.gamma / fma_rn(Q.norm_A, Q.norm_x, Q.norm_pb) <= a.tol);
-                    bool stop = false;
-                    if (it > 0 && (it % 4) == 0) {
-                        if (Q.snap0 || Q.snap1) {
-                            stop = true;
-                            Q.iters = it;
-                        }
-                    } else if (((it + 1) % 4) == 0) {
-                        Q.snap0 = Q.test0;
-                        Q.snap1 = Q.test1;
-                    }
-                    if (!isfinite(Q.inv_beta) || !isfinite(Q.inv_rho) || !isfinite(Q.eta) ||
-                        !isfinite(Q.inv_delta) || !isfinite(Q.alpha)) {
-                        Q.breakdown = 1;
-                        stop = true;
-                        Q.iters = it;
-                    }
-                    if (!stop && it + 1 >= a.max_it) Q.iters = a.max_it;
-                    if (stop) {
-                        Q.done = 1;
-                        Q.stop_it = it;
-                    }
+                    if (S[j].done) continue;
+                    scal_after_ut(S[j], r[j], r[NR + j], r[2 * NR + j], r[3 * NR + j], it, k1, a.tol, a.max_it);
                 }
             __syncthreads();
         }
@@ -1565,14 +1578,46 @@ __global__ void __launch_bounds__(kT, kCtasPerSm) k_sqmr_many(const PArgs<TF>* _
     }
 }
 
-// The instantiations, one translation unit each (sqmr_kernels_*.cu): every
-// body takes the compiler some twenty seconds.
-#define CULIPX_SQMR_PERSISTENT(X, TF, NR)                       \
-    X template __global__ void k_sqmr_persistent<TF, 1, NR>(PArgs<TF>); \
-    X template __global__ void k_sqmr_persistent<TF, 2, NR>(PArgs<TF>);
-#define CULIPX_SQMR_BATCHED(X, TF) X template __global__ void k_sqmr_batched<TF>(PArgs<TF>, BatchArgs);
-#define CULIPX_SQMR_MANY(X, TF, MULTI) \
-    X template __global__ void k_sqmr_many<TF, MULTI>(const PArgs<TF>* __restrict__, const int* __restrict__, int, int*);
+// The kernels' addresses.  Each is defined in one translation unit of its own
+// (sqmr_kernels_*.cu): every body takes the compiler some twenty seconds.
+template <class TF, int CTAS, int NR>
+const void* persistent_fn();
+template <class TF>
+const void* batched_fn();
+template <class TF, bool MULTI>
+const void* many_fn();
+
+#define CULIPX_SQMR_DECLARE(TF)                            \
+    template <> const void* persistent_fn<TF, 1, 1>();     \
+    template <> const void* persistent_fn<TF, 2, 1>();     \
+    template <> const void* persistent_fn<TF, 1, 2>();     \
+    template <> const void* persistent_fn<TF, 2, 2>();     \
+    template <> const void* persistent_fn<TF, 1, 4>();     \
+    template <> const void* persistent_fn<TF, 2, 4>();     \
+    template <> const void* batched_fn<TF>();              \
+    template <> const void* many_fn<TF, false>();          \
+    template <> const void* many_fn<TF, true>();
+CULIPX_SQMR_DECLARE(double)
+CULIPX_SQMR_DECLARE(float)
+
+#define CULIPX_SQMR_PERSISTENT(TF, CTAS, NR)          \
+    template <>                                       \
+    const void* persistent_fn<TF, CTAS, NR>()         \
+    {                                                 \
+        return (const void*)k_sqmr_persistent<TF, CTAS, NR>; \
+    }
+#define CULIPX_SQMR_BATCHED(TF)                \
+    template <>                                \
+    const void* batched_fn<TF>()               \
+    {                                          \
+        return (const void*)k_sqmr_batched<TF>; \
+    }
+#define CULIPX_SQMR_MANY(TF, MULTI)                \
+    template <>                                    \
+    const void* many_fn<TF, MULTI>()               \
+    {                                              \
+        return (const void*)k_sqmr_many<TF, MULTI>; \
+    }
 
 }  // namespace persistent
 

@@ -239,3 +239,28 @@ def test_batch_factor_solve_graph_replays_bit_for_bit(precision):
         assert torch.equal(x, x2), call
         for k in ("val", "tri", "perm"):
             assert np.array_equal(F.export()[k], F2.export()[k]), (call, k)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", [cb.F64, cb.F32])
+@pytest.mark.parametrize("block", [16, 32])
+def test_batch_same_bits_on_the_whole_grid_and_on_one_cta(precision, block):
+    """A batch with a large system iterates on the whole grid, one of small
+    systems gives each a CTA: a small system's result is the same bits in
+    both, as are all results whatever stands around them."""
+    h = cb.Handle(0)
+    small = _systems(5, seed=31)
+    n = 6400
+    rp, ci, v = cb.kkt_generate(n, n // 2, 6, 16, 1e-2, 1e2, seed=77)
+    large = (rp, ci, v, cb.kkt_blocking(n, n // 2, block))
+    tiny = [(r, c, w, cb.kkt_blocking(40, 3, 2)) for r, c, w in [cb.kkt_generate(40, 3, 2, 0, 1e-1, 1e1, seed=5)]]
+    syst = small[:3] + [large] + tiny + small[3:]
+    rhs = _rhs(syst, range(7))
+    x, res, its, st, off, _ = _solve_batch(h, syst, precision, max_it=40, rhs=rhs)
+    alone = syst[:3] + syst[4:]
+    xa, resa, itsa, sta, offa, _ = _solve_batch(h, alone, precision, max_it=40, rhs=rhs[:3] + rhs[4:])
+    for j, k in enumerate([0, 1, 2, 4, 5, 6]):
+        assert its[k] == itsa[j] and res[k] == resa[j] and st[k] == sta[j]
+        assert np.array_equal(x[off[k]:off[k + 1]], xa[offa[j]:offa[j + 1]])
+    xl, resl, itsl, stl, _, _ = _solve_batch(h, [large], precision, max_it=40, rhs=[rhs[3]])
+    assert its[3] == itsl[0] and res[3] == resl[0] and np.array_equal(x[off[3]:off[4]], xl)
