@@ -1060,6 +1060,7 @@ int factor_compute(Factor* f, const void* d_vals, const int* h_is_piv, int pivot
         f->computed = true;
         return CULIPX_OK;
     }
+    CULIPX_TRY(block_mirror(p));
     CULIPX_TRY(block_storage(f));
     CULIPX_CUDA(cudaMemsetAsync(f->val.get(), 0, p.val_slots * f->vbytes, s));
     CULIPX_CUDA(cudaMemcpyAsync(f->idx.get(), p.d_idx_init.get(), p.val_slots * sizeof(int),

@@ -5,6 +5,7 @@
 #include "common.h"
 #include "device.h"
 
+#include <mutex>
 #include <vector>
 
 namespace culipx {
@@ -77,14 +78,16 @@ struct Pattern {
     // value-store layout (level-list order)
     std::vector<BlockDesc> desc;
     long long val_slots = 0;
-    // K entry -> value slot (dense: val_off + local; sparse: val_off + running count); -1: lower
-    std::vector<int> a_dst;
-    std::vector<int> idx_init;   // val_slots entries: sparse local indices of A's entries (-1 unused)
-    std::vector<int> nnz_init;   // per block
 
-    DeviceBuffer d_row_offdiag_start, d_lvl_off;
-    DeviceBuffer d_cs_off, d_desc, d_bs, d_csc_off, d_csc_blk, d_lb, d_lvl_rows, d_a_dst, d_idx_init,
-        d_nnz_init, d_fmt, d_maxnnz, d_row_block;
+    DeviceBuffer d_lvl_off, d_lvl_rows, d_bs;
+    // what the general factorization reads (block_mirror)
+    DeviceBuffer d_row_offdiag_start, d_cs_off, d_desc, d_csc_off, d_csc_blk, d_lb, d_a_dst, d_idx_init,
+        d_nnz_init, d_fmt, d_maxnnz;
+    // two_level: K's structure, from which block_mirror builds those once a
+    // factor of the pattern first takes the general path
+    std::vector<int> k_rowptr, k_colidx;
+    std::mutex mirror_lock;
+    bool mirrored = false;
     // two_level, parts of d_two: K's row offsets; the level-0 fine rows; the
     // columns of U's entries, row after row; the entries of U', level-1 row
     // after level-1 row; K's own entries of the level-1 pivot tiles with their
@@ -101,6 +104,10 @@ struct Pattern {
 int analyze_pattern(culipx_handle_t* h, int n, const int* rowptr, const int* colidx,
                     int num_blocks, const int* block_starts, int fill_level, double fill_factor,
                     int precision, Pattern** out, int num_systems = 1, const int* system_row_offsets = nullptr);
+
+// The device arrays of the general factorization: uploaded with the analysis,
+// for a two-level pattern on the first call that needs them.
+int block_mirror(Pattern& p);
 
 }  // namespace culipx
 

@@ -434,34 +434,6 @@ int analyze_pattern(culipx_handle_t* h, int n, const int* rowptr, const int* col
         p.val_slots = o;
     }
 
-    // gather destinations of A's upper entries
-    p.a_dst.assign(p.nnz, -1);
-    p.idx_init.assign(p.val_slots, -1);
-    p.nnz_init.assign(cnz, 0);
-#pragma omp parallel for schedule(dynamic, 64)
-    for (int I = 0; I < cm; ++I) {  // a block row's slots are its own
-        const int* cb = p.cs_col.data() + p.cs_off[I];
-        const int clen = p.cs_off[I + 1] - p.cs_off[I];
-        for (int i = p.bs[I]; i < p.bs[I + 1]; ++i)
-            for (int q = rowptr[i]; q < rowptr[i + 1]; ++q) {
-                const int c = colidx[q];
-                if (c < i) continue;
-                const int J = p.row_block[c];
-                const int pos = (int)(std::lower_bound(cb, cb + clen, J) - cb);
-                const int b = p.cs_off[I] + pos;
-                const int w = blk_size(p, J);
-                const int local = (i - p.bs[I]) * w + (c - p.bs[J]);
-                const BlockDesc& d = p.desc[b];
-                if (p.fmt[b] == kDense) {
-                    p.a_dst[q] = d.val_off + local;
-                } else {
-                    const int slot = d.val_off + p.nnz_init[b]++;
-                    p.a_dst[q] = slot;
-                    p.idx_init[slot] = local;
-                }
-            }
-    }
-
     TwoLevel two;
     p.two_level = two_level_form(p, rowptr, colidx, two);
 
@@ -474,21 +446,13 @@ int analyze_pattern(culipx_handle_t* h, int n, const int* rowptr, const int* col
     auto up = [&](DeviceBuffer& buf, const void* src, size_t bytes) {
         if (st == CULIPX_OK) st = buf.upload(h, src, bytes);
     };
-    up(p.d_cs_off, p.cs_off.data(), sizeof(int) * (cm + 1));
-    up(p.d_row_offdiag_start, p.row_offdiag_start.data(), sizeof(int) * cm);
     up(p.d_lvl_off, p.lvl_off.data(), sizeof(int) * (p.num_levels + 1));
-    up(p.d_desc, p.desc.data(), sizeof(BlockDesc) * cnz);
-    up(p.d_bs, p.bs.data(), sizeof(int) * (cm + 1));
-    up(p.d_csc_off, p.csc_off.data(), sizeof(int) * (cm + 1));
-    up(p.d_csc_blk, p.csc_blk.data(), sizeof(int) * cnz);
-    up(p.d_lb, p.lb.data(), sizeof(int) * cnz);
     up(p.d_lvl_rows, p.lvl_rows.data(), sizeof(int) * cm);
-    up(p.d_a_dst, p.a_dst.data(), sizeof(int) * p.nnz);
-    up(p.d_idx_init, p.idx_init.data(), sizeof(int) * p.val_slots);
-    up(p.d_nnz_init, p.nnz_init.data(), sizeof(int) * cnz);
-    up(p.d_fmt, p.fmt.data(), sizeof(int) * cnz);
-    up(p.d_maxnnz, p.max_nnz.data(), sizeof(int) * cnz);
-    up(p.d_row_block, p.row_block.data(), sizeof(int) * n);
+    up(p.d_bs, p.bs.data(), sizeof(int) * (cm + 1));
+    p.device_bytes = (long long)(p.d_lvl_off.bytes() + p.d_lvl_rows.bytes() + p.d_bs.bytes());
+    p.k_rowptr.assign(rowptr, rowptr + n + 1);
+    p.k_colidx.assign(colidx, colidx + p.nnz);
+    if (!p.two_level && st == CULIPX_OK) st = block_mirror(p);
     if (p.two_level) {
         // one allocation and copy for all of them, each part on a 16-byte boundary
         const std::pair<const void*, size_t> parts[] = {
@@ -522,10 +486,65 @@ int analyze_pattern(culipx_handle_t* h, int n, const int* rowptr, const int* col
         p.two_l0_scan = reinterpret_cast<const int*>(d + at[7]);
     }
     if (st != CULIPX_OK) { delete pp; return st; }
-    p.device_bytes = (long long)(p.d_cs_off.bytes() + p.d_desc.bytes() + p.d_bs.bytes() + p.d_csc_off.bytes() + p.d_csc_blk.bytes() +
-                                 p.d_lb.bytes() + p.d_lvl_rows.bytes() + p.d_a_dst.bytes() + p.d_idx_init.bytes() +
-                                 p.d_nnz_init.bytes() + p.d_fmt.bytes() + p.d_maxnnz.bytes() + p.d_row_block.bytes() + p.d_two.bytes());
+    p.device_bytes += (long long)p.d_two.bytes();
     *out = pp;
+    return CULIPX_OK;
+}
+
+int block_mirror(Pattern& p)
+{
+    std::lock_guard<std::mutex> lock(p.mirror_lock);
+    if (p.mirrored) return CULIPX_OK;
+    culipx_handle_t* h = p.handle;
+    const int cm = p.num_blocks, cnz = p.coarse_nnz;
+    // gather destinations of A's upper entries
+    std::vector<int> a_dst(p.nnz, -1), idx_init(p.val_slots, -1), nnz_init(cnz, 0);
+#pragma omp parallel for schedule(dynamic, 64)
+    for (int I = 0; I < cm; ++I) {  // a block row's slots are its own
+        const int* cb = p.cs_col.data() + p.cs_off[I];
+        const int clen = p.cs_off[I + 1] - p.cs_off[I];
+        for (int i = p.bs[I]; i < p.bs[I + 1]; ++i)
+            for (int q = p.k_rowptr[i]; q < p.k_rowptr[i + 1]; ++q) {
+                const int c = p.k_colidx[q];
+                if (c < i) continue;
+                const int J = p.row_block[c];
+                const int pos = (int)(std::lower_bound(cb, cb + clen, J) - cb);
+                const int b = p.cs_off[I] + pos;
+                const int w = blk_size(p, J);
+                const int local = (i - p.bs[I]) * w + (c - p.bs[J]);
+                const BlockDesc& d = p.desc[b];
+                if (p.fmt[b] == kDense) {
+                    a_dst[q] = d.val_off + local;
+                } else {
+                    const int slot = d.val_off + nnz_init[b]++;
+                    a_dst[q] = slot;
+                    idx_init[slot] = local;
+                }
+            }
+    }
+
+    long long bytes = 0;
+    auto up = [&](DeviceBuffer& buf, const void* src, size_t size) -> int {
+        if (buf.get()) return CULIPX_OK;  // an earlier call that ran out of memory got this far
+        CULIPX_TRY(buf.upload(h, src, size));
+        bytes += (long long)buf.bytes();
+        return CULIPX_OK;
+    };
+    CULIPX_TRY(up(p.d_cs_off, p.cs_off.data(), sizeof(int) * (cm + 1)));
+    CULIPX_TRY(up(p.d_row_offdiag_start, p.row_offdiag_start.data(), sizeof(int) * cm));
+    CULIPX_TRY(up(p.d_desc, p.desc.data(), sizeof(BlockDesc) * cnz));
+    CULIPX_TRY(up(p.d_csc_off, p.csc_off.data(), sizeof(int) * (cm + 1)));
+    CULIPX_TRY(up(p.d_csc_blk, p.csc_blk.data(), sizeof(int) * cnz));
+    CULIPX_TRY(up(p.d_lb, p.lb.data(), sizeof(int) * cnz));
+    CULIPX_TRY(up(p.d_a_dst, a_dst.data(), sizeof(int) * p.nnz));
+    CULIPX_TRY(up(p.d_idx_init, idx_init.data(), sizeof(int) * p.val_slots));
+    CULIPX_TRY(up(p.d_nnz_init, nnz_init.data(), sizeof(int) * cnz));
+    CULIPX_TRY(up(p.d_fmt, p.fmt.data(), sizeof(int) * cnz));
+    CULIPX_TRY(up(p.d_maxnnz, p.max_nnz.data(), sizeof(int) * cnz));
+    p.device_bytes += bytes;
+    p.k_rowptr = std::vector<int>();
+    p.k_colidx = std::vector<int>();
+    p.mirrored = true;
     return CULIPX_OK;
 }
 
