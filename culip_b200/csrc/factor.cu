@@ -1004,19 +1004,9 @@ int factor_create(Pattern* p, Factor** out)
         al(f->u_pair, 2 * (size_t)p->two_entries * f->vbytes);
     }
     al(f->work, (size_t)n * f->vbytes);
-    {
-        // packed pivot tile triangles: h_I (h_I + 1) / 2 slots per block row,
-        // rounded up to 4 slots so that every tile starts on a 16-byte
-        // boundary (16-byte asynchronous copies into shared memory)
-        std::vector<long long> pko(cm + 1, 0);
-        for (int I = 0; I < cm; ++I) {
-            const long long hI = p->bs[I + 1] - p->bs[I];
-            pko[I + 1] = pko[I] + (hI * (hI + 1) / 2 + 3) / 4 * 4;
-        }
-        if (st == CULIPX_OK) st = f->pk_off.upload(h, pko.data(), (cm + 1) * sizeof(long long));
-        al(f->pk_col, (size_t)pko[cm] * f->vbytes);
-        al(f->pk_row, (size_t)pko[cm] * f->vbytes);
-    }
+    if (st == CULIPX_OK) st = f->pk_off.upload(h, p->pk_off.data(), (cm + 1) * sizeof(long long));
+    al(f->pk_col, (size_t)p->pk_off[cm] * f->vbytes);
+    al(f->pk_row, (size_t)p->pk_off[cm] * f->vbytes);
     al(f->ndmask, cm * sizeof(unsigned));
     al(f->scan_s, (cm + 1) * sizeof(int));
     al(f->scan_c, (cm + 1) * sizeof(int));
@@ -1173,10 +1163,9 @@ int export_two_level(Factor* f, int* blk_nnz, long long* blk_off, int* idx, void
     const size_t vb = f->vbytes;
     std::vector<int2> rng(n);
     std::vector<int> flags(cm);
-    std::vector<long long> pko(cm + 1);
+    const std::vector<long long>& pko = p.pk_off;
     CULIPX_CUDA(cudaMemcpyAsync(rng.data(), f->u_rng.get(), n * sizeof(int2), cudaMemcpyDeviceToHost, s));
     CULIPX_CUDA(cudaMemcpyAsync(flags.data(), f->rowflags.get(), cm * sizeof(int), cudaMemcpyDeviceToHost, s));
-    CULIPX_CUDA(cudaMemcpyAsync(pko.data(), f->pk_off.get(), (cm + 1) * sizeof(long long), cudaMemcpyDeviceToHost, s));
     CULIPX_CUDA(cudaStreamSynchronize(s));
     int slots = 0;
     for (const int2& r : rng) slots = std::max(slots, r.y);

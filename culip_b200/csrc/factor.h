@@ -112,6 +112,8 @@ int factor_export(Factor* f, int* blk_nnz, long long* blk_off, int* idx, void* v
 // factor.cu's launch sequence and build_sweeps in three launches, for patterns
 // with Pattern::two_level under BK / Rook pivoting without a drop threshold
 int factor_two_level(Factor* f, const void* d_vals, cudaStream_t stream, int* launches);
+// prec_apply's triangular stages for such a factor (apply_two_level.cu)
+int two_level_apply(Factor* f, bool left, const void* d_b, void* d_x, cudaStream_t stream);
 int prec_apply(Factor* f, int stage, const void* d_b, void* d_x, cudaStream_t stream);
 
 }  // namespace culipx

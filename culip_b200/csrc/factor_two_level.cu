@@ -29,6 +29,7 @@
 // 256 systems of 2.0 M rows in FP32: 0.57 ms against 3.4.
 #include "factor.h"
 #include "kernels_common.cuh"
+#include "launch.cuh"
 #include "pivot_tile.cuh"
 
 #include <algorithm>
@@ -55,7 +56,6 @@ template <class T>
 struct TwoArgs {
     int n0;               // level-0 fine rows
     int q1, nr1;          // first position of level 1 in lvl_rows, its block rows
-    int entries;          // of U, dropped ones included
     int method;
     double piv64;
     const T* kval;
@@ -65,6 +65,7 @@ struct TwoArgs {
     const int* ucol;
     const int2* low;
     const int2* tail;
+    const two::Tile* tiles;
     const int* tail_off;
     const int* slot;
     const int* l0_scan;
@@ -115,11 +116,16 @@ template <class T>
 __global__ void __launch_bounds__(256) k_two_rows(TwoArgs<T> a)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    int tagged = 0, g = 0, k0 = 0, k1 = 0, o0 = 0;
+    if (i < a.n0) {
+        tagged = __ldg(a.l0_rows + i);
+        g = tagged & two::kRowMask;
+        k0 = __ldg(a.kp + g);
+        k1 = __ldg(a.kp + g + 1);
+        o0 = __ldg(a.slot + g);
+    }
+    after_previous();  // K's values; what stands above is the pattern's
     if (i >= a.n0) return;
-    const int tagged = __ldg(a.l0_rows + i);
-    const int g = tagged & two::kRowMask;
-    const int k0 = __ldg(a.kp + g), k1 = __ldg(a.kp + g + 1);
-    const int o0 = __ldg(a.slot + g);
     const T d11 = level0_pivot(a, tagged, k0);
     const T d22 = (tagged & two::kNextInBlock) ? level0_pivot(a, __ldg(a.l0_rows + i + 1), k1) : T(0);
     const T d12 = T(0);
@@ -205,20 +211,23 @@ __global__ void __launch_bounds__(32 * kTileWarps) k_two_tiles(TwoArgs<T> a)
     __shared__ int piv_s[kTileWarps][32];
     const int warp = threadIdx.x >> 5;
     const int t = blockIdx.x * kTileWarps + warp;
-    if (t >= a.nr1) return;
+    if (t >= a.nr1) {
+        after_previous();
+        return;
+    }
     const int b = lane_id();
     T* tile = tiles[warp];
-    const int I = __ldg(a.lvl_rows + a.q1 + t);
-    const int fr = __ldg(a.bs + I), h = __ldg(a.bs + I + 1) - fr;
+    const int4* td = reinterpret_cast<const int4*>(a.tiles + t);
+    const int4 d0 = __ldg(td), d1 = __ldg(td + 1);
+    const int I = d0.x, fr = d0.y, h = d0.z;
     const int me = fr + b;
     int k0 = 0, k1 = 0;
     if (b < h) {
         k0 = __ldg(a.slot + me);
-        // the rows' lists follow each other in level order, the last one ends with U
-        if (b + 1 < h) k1 = __ldg(a.slot + me + 1);
-        else k1 = (t + 1 < a.nr1) ? __ldg(a.slot + __ldg(a.bs + __ldg(a.lvl_rows + a.q1 + t + 1))) : a.entries;
+        k1 = (b + 1 < h) ? __ldg(a.slot + me + 1) : d1.x + d0.w;
     }
     for (int e = b; e < kTileElems; e += 32) tile[e] = T(0);
+    after_previous();  // the rows of U; what stands above is the pattern's
     __syncwarp();
     for (int k = __ldg(a.tail_off + t) + b; k < __ldg(a.tail_off + t + 1); k += 32) {
         const int2 e = __ldg(a.tail + k);
@@ -273,6 +282,11 @@ __global__ void __launch_bounds__(32 * kTileWarps) k_two_tiles(TwoArgs<T> a)
         cur = nxt;
     }
     subtract();
+    // the sweeps read a tile's run of slots whole
+    for (int q = ut; q < k1; ++q) {
+        a.ut_col[q] = 0;
+        a.ut_val[q] = T(0);
+    }
     __syncwarp();
 
     int* perm = perm_s[warp];
@@ -324,8 +338,9 @@ __global__ void __launch_bounds__(32 * kTileWarps) k_two_tiles(TwoArgs<T> a)
     // a 2x2 pivot's rounding residue left of its second row's diagonal, for the export
     if (two && b < h) a.u_sub[me] = b > 0 ? tile[b * kTileStride + b - 1] : T(0);
     if (!ident) {
-        T* pc = a.pk_col + __ldg(a.pk_off + I);
-        T* pr = a.pk_row + __ldg(a.pk_off + I);
+        const long long pko = ((long long)d1.w << 32) | (unsigned)d1.z;
+        T* pc = a.pk_col + pko;
+        T* pr = a.pk_row + pko;
         for (int r = 0; r < h; ++r)
             if (b >= r && b < h) {
                 const T v = tile[r * kTileStride + b];
@@ -425,6 +440,7 @@ __device__ void split_rows(const TwoArgs<T>& a, int q0)
 template <class T>
 __global__ void __launch_bounds__(kOrderT) k_two_order(TwoArgs<T> a, int splits)
 {
+    after_previous();
     if ((int)blockIdx.x < splits) {
         split_rows(a, blockIdx.x * kOrderT);
         return;
@@ -498,13 +514,13 @@ int run(Factor* f, const void* d_vals, cudaStream_t s, int* launches)
     a.nr1 = p.lvl_off[2] - p.lvl_off[1];
     a.method = f->pivot;
     a.piv64 = f->pivot_fp64;
-    a.entries = p.two_entries;
     a.kval = static_cast<const T*>(d_vals);
     a.kp = p.two_kp;
     a.l0_rows = p.two_l0_rows;
     a.ucol = p.two_ucol;
     a.low = p.two_low;
     a.tail = p.two_tail;
+    a.tiles = p.two_tiles;
     a.tail_off = p.two_tail_off;
     a.up = f->u_pair.as<typename Pair<T>::type>();
     a.slot = p.two_slot;
@@ -535,12 +551,14 @@ int run(Factor* f, const void* d_vals, cudaStream_t s, int* launches)
     a.cplx = f->cplx.as<int>();
     a.citem = f->citem.as<CItem>();
     a.kind = f->kind.as<unsigned char>();
-    k_two_rows<T><<<(a.n0 + 255) / 256, 256, 0, s>>>(a);
-    k_two_tiles<T><<<(a.nr1 + kTileWarps - 1) / kTileWarps, 32 * kTileWarps, 0, s>>>(a);
+    CULIPX_TRY(launch_overlapped(k_two_rows<T>, dim3((a.n0 + 255) / 256), dim3(256), s, !f->capturing, a));
+    CULIPX_TRY(launch_overlapped(k_two_tiles<T>, dim3((a.nr1 + kTileWarps - 1) / kTileWarps), dim3(32 * kTileWarps),
+                                 s, !f->capturing, a));
     const int splits = (a.nr1 + kOrderT - 1) / kOrderT;
-    k_two_order<T><<<(a.n0 + kOrderT - 1) / kOrderT + splits, kOrderT, 0, s>>>(a, splits);
+    CULIPX_TRY(launch_overlapped(k_two_order<T>, dim3((a.n0 + kOrderT - 1) / kOrderT + splits), dim3(kOrderT), s,
+                                 !f->capturing, a, splits));
     *launches += 3;
-    return launch_check("two-level factorization");
+    return CULIPX_OK;
 }
 
 }  // namespace

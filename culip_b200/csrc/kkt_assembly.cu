@@ -20,6 +20,7 @@
 // once: nnz_K (8 + 8) + 8 nnz_A + 16 n bytes (HBM-bound).
 #include "kkt_assembly.h"
 #include "kernels_common.cuh"
+#include "launch.cuh"
 
 #include <algorithm>
 #include <vector>
@@ -34,6 +35,7 @@ __global__ void k_kkt_values(long long nnz_k, int n, const long long* __restrict
                              const double* __restrict__ s, const double* __restrict__ d, double delta, double gamma,
                              TO* __restrict__ kval)
 {
+    after_previous();
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < nnz_k; e += stride) {
         const long long q = __ldg(src + e);
@@ -141,14 +143,15 @@ int kkt_assembly_values(KktAssembly* K, const double* d_aval, const double* d_x,
     cudaStream_t s = K->handle->stream;
     const long long blocks = std::min<long long>((K->nnz_k + 255) / 256, 148LL * 8);
     if (blocks <= 0) return CULIPX_OK;
+    const dim3 grid((unsigned)blocks), block(256);
     if (precision == CULIPX_F64)
-        k_kkt_values<double><<<(unsigned)blocks, 256, 0, s>>>(K->nnz_k, K->n, K->src.as<long long>(), d_aval, d_x, d_s,
-                                                              d_d, delta, gamma, static_cast<double*>(d_kval));
+        CULIPX_TRY(launch_overlapped(k_kkt_values<double>, grid, block, s, true, K->nnz_k, K->n, K->src.as<long long>(),
+                                     d_aval, d_x, d_s, d_d, delta, gamma, static_cast<double*>(d_kval)));
     else
-        k_kkt_values<float><<<(unsigned)blocks, 256, 0, s>>>(K->nnz_k, K->n, K->src.as<long long>(), d_aval, d_x, d_s,
-                                                             d_d, delta, gamma, static_cast<float*>(d_kval));
+        CULIPX_TRY(launch_overlapped(k_kkt_values<float>, grid, block, s, true, K->nnz_k, K->n, K->src.as<long long>(),
+                                     d_aval, d_x, d_s, d_d, delta, gamma, static_cast<float*>(d_kval)));
     K->handle->launches += 1;
-    return launch_check("k_kkt_values");
+    return CULIPX_OK;
 }
 
 }  // namespace culipx

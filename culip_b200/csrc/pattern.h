@@ -31,6 +31,15 @@ constexpr int kColMask = 0x7fffffff;
 constexpr int kSameBlock = (int)0x80000000u;  // low.x: same block row as the entry before it
 constexpr int kBeforeShift = 27;              // low.y: entries of the same row and tile before it, over
 constexpr int kSlotMask = (1 << 27) - 1;      //        its slot in U
+
+// a level-1 block row: its rows, its rows' run of entries of U', the place of
+// its packed pivot triangles (two 16-byte loads)
+struct alignas(16) Tile {
+    int I, fr, h, entries;
+    int slot, pad;
+    long long pk_off;
+};
+static_assert(sizeof(Tile) == 32, "Tile is two 16-byte words");
 }  // namespace two
 
 struct Pattern {
@@ -66,6 +75,9 @@ struct Pattern {
     bool two_level = false;
     int l0_count = 0;             // fine rows of level 0
     int two_entries = 0;          // entries of U
+    // slots of the pivot tiles' packed triangles (h_I (h_I + 1) / 2 per block
+    // row, rounded up to 4 slots: every tile on a 16-byte boundary)
+    std::vector<long long> pk_off;
     std::vector<int> lb_off, lb;  // factor order per level: pivots, then off-diagonal (CSR order)
     // per row position t of lvl_rows: index of the row's first off-diagonal
     // block inside its level's off-diagonal list
@@ -88,7 +100,7 @@ struct Pattern {
     std::vector<int> k_rowptr, k_colidx;
     std::mutex mirror_lock;
     bool mirrored = false;
-    // two_level, parts of d_two: K's row offsets; the level-0 fine rows; the
+    // two_level, parts of d_two: the level-1 block rows; K's row offsets; the level-0 fine rows; the
     // columns of U's entries, row after row; the entries of U', level-1 row
     // after level-1 row; K's own entries of the level-1 pivot tiles with their
     // offsets per tile; per fine row its first entry in U (level 0) or U'
@@ -96,6 +108,7 @@ struct Pattern {
     DeviceBuffer d_two;
     const int *two_kp = nullptr, *two_l0_rows = nullptr, *two_ucol = nullptr, *two_tail_off = nullptr,
               *two_slot = nullptr, *two_l0_scan = nullptr;
+    const two::Tile* two_tiles = nullptr;
     const int2 *two_low = nullptr, *two_tail = nullptr;
     long long device_bytes = 0;
 };

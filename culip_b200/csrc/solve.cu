@@ -20,6 +20,7 @@
 #include "factor.h"
 #include "kernels_common.cuh"
 #include "block_io.cuh"
+#include "launch.cuh"
 
 #include <algorithm>
 
@@ -646,16 +647,20 @@ __device__ __forceinline__ void givens_solve(C p11, C p12, C p22, C r1, C r2, C&
     g1 = fma_rn(-tp12, g2, g1) / gr;
 }
 
-// k_solve_D: Givens-based 1x1 / 2x2 block-diagonal solve (out may equal in);
+// k_solve_D: Givens-based 1x1 / 2x2 block-diagonal solve (out may equal in),
+// D's diagonal from its own array (tri holds three values a row: 1.5 M rows in
+// FP32 12.3 us with it alone);
 // an FP32 factor's ill-conditioned 2x2 pivots (wide_2x2) are solved in FP64
 template <class T>
-__global__ void k_solve_D(const T* __restrict__ tri, const int* __restrict__ is_piv, const T* in, T* out, int n,
-                          double piv64)
+__global__ void k_solve_D(const T* __restrict__ tri, const T* __restrict__ dg, const int* __restrict__ is_piv,
+                          const T* in, T* out, int n, double piv64)
 {
+    after_previous();
     for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < n; g += gridDim.x * blockDim.x) {
         const int this_piv = is_piv[g];
         const int next_piv = (g < n - 1) ? is_piv[g + 1] : 1;
-        const T p11 = tri[3 * (size_t)g + 1], p12 = tri[3 * (size_t)g + 2];
+        // no coupling is stored right of a row that a 1x1 pivot follows
+        const T p11 = dg[g], p12 = !next_piv ? tri[3 * (size_t)g + 2] : T(0);
         const T p22 = !next_piv ? tri[3 * (size_t)(g + 1) + 1] : T(1);
         const T r1 = in[g], r2 = (g < n - 1) ? in[g + 1] : T(0);
         T g1, g2;
@@ -744,8 +749,8 @@ int apply_t(Factor* f, int stage, const void* d_b, void* d_x, cudaStream_t s)
     T* x = static_cast<T*>(d_x);
     const int grid_n = (n + 255) / 256 < 148 * 8 ? (n + 255) / 256 : 148 * 8;
     if (stage == CULIPX_MIDDLE) {
-        k_solve_D<T><<<grid_n, 256, 0, s>>>(f->tri.as<T>(), f->is_piv.as<int>(), b, x, n, f->pivot_fp64);
-        return launch_check("k_solve_D");
+        return launch_overlapped(k_solve_D<T>, dim3(grid_n), dim3(256), s, true, f->tri.as<T>(), f->dg.as<T>(),
+                                 f->is_piv.as<int>(), b, x, n, f->pivot_fp64);
     }
     if (f->solve_algorithm == CULIPX_SOLVE_JACOBI) {
         // x = 0, then `sweeps` block-Jacobi sweeps on the right-hand side rhs
@@ -831,9 +836,12 @@ int prec_apply(Factor* f, int stage, const void* d_b, void* d_x, cudaStream_t s)
     if (!d_b || !d_x) return fail(CULIPX_INVALID_ARG, "culipx_prec_apply: null vector");
     if (stage < CULIPX_LEFT || stage > CULIPX_RIGHT) return fail(CULIPX_INVALID_ARG, "culipx_prec_apply: bad stage");
     Pattern& p = *f->pat;
+    const bool fine = f->two_level && stage != CULIPX_MIDDLE && f->solve_algorithm != CULIPX_SOLVE_JACOBI;
     if (stage == CULIPX_MIDDLE) p.handle->launches += 1;
+    else if (fine) p.handle->launches += (stage == CULIPX_LEFT) ? 1 : 2;
     else if (f->solve_algorithm == CULIPX_SOLVE_JACOBI) p.handle->launches += f->jacobi_sweeps + 1 + (stage == CULIPX_LEFT);
     else p.handle->launches += p.num_levels + ((stage == CULIPX_LEFT && d_b == d_x) ? 1 : 0);
+    if (fine) return two_level_apply(f, stage == CULIPX_LEFT, d_b, d_x, s);
     if (f->precision == CULIPX_F64) return apply_t<double>(f, stage, d_b, d_x, s);
     return apply_t<float>(f, stage, d_b, d_x, s);
 }

@@ -21,6 +21,7 @@
 // row, with the warp's index and value loads contiguous (see Sell in spmv.h).
 #include "spmv.h"
 #include "kernels_common.cuh"
+#include "launch.cuh"
 
 #include <algorithm>
 #include <vector>
@@ -34,6 +35,7 @@ __global__ void __launch_bounds__(256) k_csr_spmv(int m, const int* __restrict__
                                                   const int* __restrict__ colidx, const T* __restrict__ val,
                                                   const T* __restrict__ x, T* __restrict__ y, T alpha, T beta)
 {
+    after_previous();
     constexpr int kRowsPerWarp = 32 / L;
     const int lane = lane_id();
     const int sub = lane % L;
@@ -63,6 +65,7 @@ __global__ void __launch_bounds__(256) k_csr_spmv_rows(int m, const int* __restr
                                                        const int* __restrict__ colidx, const T* __restrict__ val,
                                                        const T* __restrict__ x, T* __restrict__ y, T alpha, T beta)
 {
+    after_previous();
     const int row = blockIdx.x * blockDim.x + threadIdx.x;
     const int lane = lane_id();
     int rs = 0, re = 0;
@@ -112,7 +115,8 @@ int launch(const int* rowptr, const int* colidx, const void* val, int m, double 
     const T* xx = static_cast<const T*>(x);
     T* yy = static_cast<T*>(y);
     if (avg <= 16.0) {
-        k_csr_spmv_rows<T><<<(m + 255) / 256, 256, 0, s>>>(m, rowptr, colidx, v, xx, yy, (T)alpha, (T)beta);
+        return launch_overlapped(k_csr_spmv_rows<T>, dim3((m + 255) / 256), dim3(256), s, true, m, rowptr, colidx, v, xx, yy,
+                                 (T)alpha, (T)beta);
     } else {
         // 8 warps per block, 32 / L rows per warp
         auto grid = [&](int L) {
@@ -120,11 +124,11 @@ int launch(const int* rowptr, const int* colidx, const void* val, int m, double 
             return (int)std::min<long long>(blocks, 148LL * 16);
         };
         if (avg <= 24.0)
-            k_csr_spmv<T, 16><<<grid(16), 256, 0, s>>>(m, rowptr, colidx, v, xx, yy, (T)alpha, (T)beta);
-        else
-            k_csr_spmv<T, 32><<<grid(32), 256, 0, s>>>(m, rowptr, colidx, v, xx, yy, (T)alpha, (T)beta);
+            return launch_overlapped(k_csr_spmv<T, 16>, dim3(grid(16)), dim3(256), s, true, m, rowptr, colidx, v, xx, yy,
+                                     (T)alpha, (T)beta);
+        return launch_overlapped(k_csr_spmv<T, 32>, dim3(grid(32)), dim3(256), s, true, m, rowptr, colidx, v, xx, yy,
+                                 (T)alpha, (T)beta);
     }
-    return launch_check("k_csr_spmv");
 }
 
 // SELL-32 product: thread (slice s, lane) sums row rows[32 s + lane] over
@@ -141,6 +145,7 @@ __global__ void __launch_bounds__(128) k_sell_spmv(int nslices, const int* __res
                                                    const T* __restrict__ val, const T* __restrict__ x,
                                                    T* __restrict__ y, T alpha, T beta)
 {
+    after_previous();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     const int sl = t >> 5;
     if (sl >= nslices) return;
@@ -191,6 +196,7 @@ __global__ void __launch_bounds__(256) k_long_rows(int nlong, const int* __restr
                                                    const T* __restrict__ val, const T* __restrict__ x,
                                                    T* __restrict__ y, T alpha, T beta)
 {
+    after_previous();
     const int lane = lane_id();
     const int nw = (gridDim.x * blockDim.x) >> 5;
     for (int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < nlong; w += nw) {
@@ -223,17 +229,16 @@ int launch_sell(Csr* A, const void* x, void* y, double alpha, double beta, cudaS
     T* yy = static_cast<T*>(y);
     if (S.nslices > 0) {
         const long long threads = 32LL * S.nslices;
-        k_sell_spmv<T><<<(unsigned)((threads + 127) / 128), 128, 0, s>>>(
-            S.nslices, S.rows.as<int>(), S.slice_off.as<long long>(), S.slice_len.as<int>(), S.col.as<int>(),
-            S.val.as<T>(), xx, yy, (T)alpha, (T)beta);
-        CULIPX_TRY(launch_check("k_sell_spmv"));
+        CULIPX_TRY(launch_overlapped(k_sell_spmv<T>, dim3((unsigned)((threads + 127) / 128)), dim3(128), s, true, S.nslices,
+                                     S.rows.as<int>(), S.slice_off.as<long long>(), S.slice_len.as<int>(),
+                                     S.col.as<int>(), S.val.as<T>(), xx, yy, (T)alpha, (T)beta));
     }
     if (S.nlong > 0) {
         A->h->launches += 1;
         const int blocks = std::min((S.nlong + 7) / 8, 148 * 8);
-        k_long_rows<T><<<blocks, 256, 0, s>>>(S.nlong, S.long_rows.as<int>(), S.long_off.as<long long>(),
-                                              S.col.as<int>(), S.val.as<T>(), xx, yy, (T)alpha, (T)beta);
-        CULIPX_TRY(launch_check("k_long_rows"));
+        CULIPX_TRY(launch_overlapped(k_long_rows<T>, dim3(blocks), dim3(256), s, true, S.nlong, S.long_rows.as<int>(),
+                                     S.long_off.as<long long>(), S.col.as<int>(), S.val.as<T>(), xx, yy, (T)alpha,
+                                     (T)beta));
     }
     return CULIPX_OK;
 }

@@ -125,6 +125,7 @@ void coarse_pattern(Pattern& p, const int* rowptr, const int* colidx)
 struct TwoLevel {
     std::vector<int> l0_rows, l0_scan, slot, ucol, tail_off;
     std::vector<int2> low, tail;
+    std::vector<two::Tile> tiles;
 };
 
 // Fills the two-level form; false where the pattern has none: other than two
@@ -168,6 +169,8 @@ bool two_level_form(Pattern& p, const int* rowptr, const int* colidx, TwoLevel& 
             lower += k1 - rowptr[i];
         }
         w.tail_off.push_back((int)w.tail.size());
+        two::Tile tile = {I, fr, blk_size(p, I), lower - w.slot[fr], w.slot[fr], 0, p.pk_off[I]};
+        w.tiles.push_back(tile);
     }
     if (entries != lower || entries == 0) return false;
     p.two_entries = entries;
@@ -434,8 +437,13 @@ int analyze_pattern(culipx_handle_t* h, int n, const int* rowptr, const int* col
         p.val_slots = o;
     }
 
-    TwoLevel two;
-    p.two_level = two_level_form(p, rowptr, colidx, two);
+    p.pk_off.assign(cm + 1, 0);
+    for (int I = 0; I < cm; ++I) {
+        const long long hI = blk_size(p, I);
+        p.pk_off[I + 1] = p.pk_off[I] + (hI * (hI + 1) / 2 + 3) / 4 * 4;
+    }
+    TwoLevel form;
+    p.two_level = two_level_form(p, rowptr, colidx, form);
 
     // device mirror (not for a host-only handle)
     if (h->device < 0) {
@@ -457,13 +465,14 @@ int analyze_pattern(culipx_handle_t* h, int n, const int* rowptr, const int* col
         // one allocation and copy for all of them, each part on a 16-byte boundary
         const std::pair<const void*, size_t> parts[] = {
             {rowptr, sizeof(int) * (n + 1)},
-            {two.l0_rows.data(), sizeof(int) * two.l0_rows.size()},
-            {two.ucol.data(), sizeof(int) * two.ucol.size()},
-            {two.low.data(), sizeof(int2) * two.low.size()},
-            {two.tail.data(), sizeof(int2) * two.tail.size()},
-            {two.tail_off.data(), sizeof(int) * two.tail_off.size()},
-            {two.slot.data(), sizeof(int) * n},
-            {two.l0_scan.data(), sizeof(int) * two.l0_scan.size()}};
+            {form.l0_rows.data(), sizeof(int) * form.l0_rows.size()},
+            {form.ucol.data(), sizeof(int) * form.ucol.size()},
+            {form.low.data(), sizeof(int2) * form.low.size()},
+            {form.tail.data(), sizeof(int2) * form.tail.size()},
+            {form.tail_off.data(), sizeof(int) * form.tail_off.size()},
+            {form.slot.data(), sizeof(int) * n},
+            {form.l0_scan.data(), sizeof(int) * form.l0_scan.size()},
+            {form.tiles.data(), sizeof(two::Tile) * form.tiles.size()}};
         size_t total = 0;
         for (const auto& q : parts) total += (q.second + 15) / 16 * 16;
         std::vector<unsigned char> all(total);
@@ -484,6 +493,7 @@ int analyze_pattern(culipx_handle_t* h, int n, const int* rowptr, const int* col
         p.two_tail_off = reinterpret_cast<const int*>(d + at[5]);
         p.two_slot = reinterpret_cast<const int*>(d + at[6]);
         p.two_l0_scan = reinterpret_cast<const int*>(d + at[7]);
+        p.two_tiles = reinterpret_cast<const two::Tile*>(d + at[8]);
     }
     if (st != CULIPX_OK) { delete pp; return st; }
     p.device_bytes += (long long)p.d_two.bytes();
