@@ -64,6 +64,7 @@ struct TwoArgs {
     const int* l0_rows;
     const int* ucol;
     const int2* low;
+    const uint2* pairs;
     const int2* tail;
     const two::Tile* tiles;
     const int* tail_off;
@@ -163,50 +164,16 @@ __global__ void __launch_bounds__(256) k_two_rows(TwoArgs<T> a)
     a.simple_rows[i] = g;
 }
 
-// One entry of a level-1 row with what its update needs: its own u and D u,
-// and the two entries before it in the level-0 row (ahead of use).
+// One level-1 block row per warp, the upper triangle T_ab at tile[a][b].  Lane b
+// walks K's row fr + b for the diagonal's update and writes its row of U'; the
+// entries off the diagonal take theirs from the pattern's pair list, a lane per
+// entry, which keeps the lanes on the same path (walking a row's partners
+// instead: 5000 of 13 200 instructions a tile).
 template <class T>
-struct LowEntry {
-    int g, before, slot;
-    T u, du;
-    int c1, c2;
-    T du1, du2;
-};
-
-template <class T>
-__device__ __forceinline__ void load_low(const TwoArgs<T>& a, int2 w, LowEntry<T>& e)
+__global__ void __launch_bounds__(32 * kTileWarps, 6) k_two_tiles(TwoArgs<T> a)
 {
-    e.g = w.x;
-    e.before = (int)((unsigned)w.y >> two::kBeforeShift);
-    e.slot = w.y & two::kSlotMask;
-    const auto q = a.up[e.slot];
-    e.u = q.x;
-    e.du = q.y;
-    e.c1 = e.c2 = 0;
-    e.du1 = e.du2 = T(0);
-    if (e.before > 0) {
-        e.c1 = __ldg(a.ucol + e.slot - 1);
-        e.du1 = a.up[e.slot - 1].y;
-    }
-    if (e.before > 1) {
-        e.c2 = __ldg(a.ucol + e.slot - 2);
-        e.du2 = a.up[e.slot - 2].y;
-    }
-}
-
-// One level-1 block row per warp.  Lane b owns column b of the tile's upper
-// triangle (T_ab at tile[a][b], a <= b) and keeps the running sums of the
-// current update block in the mirrored places (tile[b][a], a < b; the
-// diagonal's in a register), so the update needs no synchronisation and the
-// tile is all the shared memory a warp holds.  The lane walks K's row fr + b:
-// each entry's column g is a level-0 row whose entries inside the tile up to
-// column b are the update's factors; they stand next to each other in U, so
-// the pattern holds the entry's place and the count before it, and the loads
-// of the next two entries are in flight while one is used.
-template <class T>
-__global__ void __launch_bounds__(32 * kTileWarps) k_two_tiles(TwoArgs<T> a)
-{
-    __shared__ T tiles[kTileWarps][kTileElems];
+    __shared__ __align__(16) T tiles[kTileWarps][kTileElems];
+    __shared__ T row_s[kTileWarps][kRowBuf];
     __shared__ int perm_s[kTileWarps][32];
     __shared__ int piv_s[kTileWarps][32];
     const int warp = threadIdx.x >> 5;
@@ -226,62 +193,100 @@ __global__ void __launch_bounds__(32 * kTileWarps) k_two_tiles(TwoArgs<T> a)
         k0 = __ldg(a.slot + me);
         k1 = (b + 1 < h) ? __ldg(a.slot + me + 1) : d1.x + d0.w;
     }
-    for (int e = b; e < kTileElems; e += 32) tile[e] = T(0);
     after_previous();  // the rows of U; what stands above is the pattern's
+
+    // The tile's entries of U' across the lanes: U' out, u and D u staged where
+    // the tile will be, the marks of entries in the block of the one before as
+    // bits; then each lane sums its row for the diagonal.
+    constexpr int CAP = 448, B = 7;
+    typename Pair<T>::type* const stage = reinterpret_cast<typename Pair<T>::type*>(tile);
+    unsigned* const marks = reinterpret_cast<unsigned*>(perm_s[warp]);
+    const int e0 = d1.x, e1 = d1.x + d0.w;
+    int ut = k1;
+    bool dropped = false;
+    const int q0 = __ldg(a.tail_off + t), q1 = __ldg(a.tail_off + t + 1);
+    row_s[warp][b] = T(0);
     __syncwarp();
-    for (int k = __ldg(a.tail_off + t) + b; k < __ldg(a.tail_off + t + 1); k += 32) {
+    for (int k = q0 + b; k < q1; k += 32) {  // K's diagonal, from which the update's sums are subtracted in turn
+        const int2 e = __ldg(a.tail + k);
+        if ((e.y >> 5) == (e.y & 31)) row_s[warp][e.y & 31] = __ldg(a.kval + e.x);
+    }
+    __syncwarp();
+    T diag = row_s[warp][b], sum = T(0);
+    for (int base = e0; base < e1; base += CAP) {
+        const int n = min(CAP, e1 - base);
+        for (int i0 = b; i0 < CAP && i0 - b < n; i0 += 32 * B) {
+            int2 w[B];
+            typename Pair<T>::type q[B];
+#pragma unroll
+            for (int j = 0; j < B; ++j) w[j] = (i0 + 32 * j < n) ? __ldg(a.low + base + i0 + 32 * j) : make_int2(0, -1);
+#pragma unroll
+            for (int j = 0; j < B; ++j)
+                if (w[j].y >= 0) q[j] = a.up[w[j].y];
+#pragma unroll
+            for (int j = 0; j < B; ++j) {
+                const unsigned m = __ballot_sync(0xffffffffu, w[j].x < 0);
+                if (b == 0 && i0 + 32 * j < n) marks[(i0 + 32 * j) / 32] = m;
+                if (w[j].y < 0) continue;
+                stage[i0 + 32 * j] = q[j];
+                a.ut_col[base + i0 + 32 * j] = w[j].x & two::kColMask;
+                a.ut_val[base + i0 + 32 * j] = q[j].x;
+                dropped |= q[j].x == T(0);
+            }
+        }
+        __syncwarp();
+        for (int e = max(k0, base); e < min(k1, base + n); ++e) {
+            const auto q = stage[e - base];
+            if (!((marks[(e - base) >> 5] >> ((e - base) & 31)) & 1u)) {  // another update block begins
+                diag -= sum;
+                sum = T(0);
+            }
+            if (q.x != T(0)) sum = fma_rn(q.x, q.y, sum);
+        }
+        __syncwarp();
+    }
+    if (__any_sync(0xffffffffu, dropped)) {  // the rows without the dropped entries
+        ut = k0;
+        for (int k = k0; k < k1; ++k) {
+            const int2 w = __ldg(a.low + k);
+            const T u = a.up[w.y].x;
+            if (u == T(0)) continue;
+            a.ut_col[ut] = w.x & two::kColMask;
+            a.ut_val[ut] = u;
+            ++ut;
+        }
+    }
+    for (int e = b; e < kTileElems; e += 32) tile[e] = T(0);
+    __syncwarp();
+    for (int k = q0 + b; k < q1; k += 32) {
         const int2 e = __ldg(a.tail + k);
         tile[(e.y >> 5) * kTileStride + (e.y & 31)] = __ldg(a.kval + e.x);
     }
     __syncwarp();
-
-    int ut = k0;
-    T pdiag = T(0);
-    unsigned touched = 0;
-    T* const col = tile + b;
-    T* const sum = tile + b * kTileStride;
-    auto subtract = [&]() {
-        while (touched) {
-            const int r = __ffs(touched) - 1;
-            touched &= touched - 1;
-            if (r == b) {
-                col[r * kTileStride] -= pdiag;
-                pdiag = T(0);
-            } else {
-                col[r * kTileStride] -= sum[r];
-                sum[r] = T(0);
+    if (b < h) tile[b * kTileStride + b] = diag - sum;
+    const int p0 = d1.y, p1 = __ldg(&a.tiles[t + 1].pair);
+    for (int i = p0 + b; i < p1; i += 32) {
+        uint2 m = __ldg(a.pairs + i);
+        if (m.x & two::kSameTarget) continue;  // its entry's first pair is another lane's
+        T* const at = tile + (m.x >> two::kPlaceShift) * kTileStride + (m.y >> two::kPlaceShift);
+        T v = *at;
+        T s = T(0);
+        auto add = [&]() {
+            const T u = a.up[m.x & two::kSlotMask].x, du = a.up[m.y & two::kSlotMask].y;
+            if (u != T(0) && du != T(0)) s = fma_rn(u, du, s);  // neither dropped
+        };
+        add();
+        for (int j = i + 1; j < p1; ++j) {
+            m = __ldg(a.pairs + j);
+            if (!(m.x & two::kSameTarget)) break;
+            if (!(m.y & two::kSameSum)) {
+                v -= s;
+                s = T(0);
             }
+            add();
         }
-    };
-    LowEntry<T> cur, nxt;
-    int2 ahead = make_int2(0, 0);
-    if (k0 < k1) load_low(a, __ldg(a.low + k0), cur);
-    if (k0 + 1 < k1) ahead = __ldg(a.low + k0 + 1);
-    for (int k = k0; k < k1; ++k) {
-        if (k + 1 < k1) load_low(a, ahead, nxt);
-        if (k + 2 < k1) ahead = __ldg(a.low + k + 2);
-        if (cur.g >= 0) subtract();  // another update block begins
-        if (cur.u != T(0)) {         // not dropped
-            a.ut_col[ut] = cur.g & two::kColMask;
-            a.ut_val[ut] = cur.u;
-            ++ut;
-            auto add = [&](int r, T du) {
-                if (du == T(0)) return;
-                touched |= 1u << r;
-                sum[r] = fma_rn(cur.u, du, sum[r]);
-            };
-            for (int q = cur.before; q > 2; --q)
-                add((__ldg(a.ucol + cur.slot - q) & two::kColMask) - fr, a.up[cur.slot - q].y);
-            if (cur.before > 1) add((cur.c2 & two::kColMask) - fr, cur.du2);
-            if (cur.before > 0) add((cur.c1 & two::kColMask) - fr, cur.du1);
-            if (cur.du != T(0)) {
-                touched |= 1u << b;
-                pdiag = fma_rn(cur.u, cur.du, pdiag);
-            }
-        }
-        cur = nxt;
+        *at = v - s;
     }
-    subtract();
     // the sweeps read a tile's run of slots whole
     for (int q = ut; q < k1; ++q) {
         a.ut_col[q] = 0;
@@ -295,9 +300,9 @@ __global__ void __launch_bounds__(32 * kTileWarps) k_two_tiles(TwoArgs<T> a)
     perm[b] = b;
     piv[b] = 1;
     __syncwarp();
-    bool diag = true;
-    for (int r = 0; r < h; ++r) diag &= b <= r || b >= h || tile[r * kTileStride + b] == T(0);
-    if (__all_sync(0xffffffffu, diag)) {
+    bool diagonal = true;
+    for (int r = 0; r < h; ++r) diagonal &= b <= r || b >= h || tile[r * kTileStride + b] == T(0);
+    if (__all_sync(0xffffffffu, diagonal)) {
         // 1x1 pivots without swaps (k_pivot_blocks' short cut)
         if (b < h) {
             T d = tile[b * kTileStride + b];
@@ -309,7 +314,7 @@ __global__ void __launch_bounds__(32 * kTileWarps) k_two_tiles(TwoArgs<T> a)
         }
         __syncwarp();
     } else {
-        factorize_tile(tile, h, piv, D, perm, a.method, a.piv64);
+        factorize_tile_window(tile, row_s[warp], h, piv, D, perm, a.method, a.piv64);
     }
     __syncwarp();
 
@@ -341,12 +346,11 @@ __global__ void __launch_bounds__(32 * kTileWarps) k_two_tiles(TwoArgs<T> a)
         const long long pko = ((long long)d1.w << 32) | (unsigned)d1.z;
         T* pc = a.pk_col + pko;
         T* pr = a.pk_row + pko;
-        for (int r = 0; r < h; ++r)
-            if (b >= r && b < h) {
-                const T v = tile[r * kTileStride + b];
-                pc[b * (b + 1) / 2 + r] = v;
-                pr[r * h - r * (r - 1) / 2 + b - r] = v;
-            }
+        // across the lanes: columns of the triangle into pc, rows into pr
+        for (int k = 0; k < h; ++k) {
+            if (b <= k) pc[k * (k + 1) / 2 + b] = tile[b * kTileStride + k];
+            if (b >= k && b < h) pr[k * h - k * (k - 1) / 2 + b - k] = tile[k * kTileStride + b];
+        }
     }
 }
 
@@ -519,6 +523,7 @@ int run(Factor* f, const void* d_vals, cudaStream_t s, int* launches)
     a.l0_rows = p.two_l0_rows;
     a.ucol = p.two_ucol;
     a.low = p.two_low;
+    a.pairs = p.two_pairs;
     a.tail = p.two_tail;
     a.tiles = p.two_tiles;
     a.tail_off = p.two_tail_off;

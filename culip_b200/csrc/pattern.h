@@ -29,14 +29,17 @@ constexpr int kRowMask = kRowDense - 1;
 constexpr int kDense = (int)0x80000000u;      // ucol: the entry is in a dense block
 constexpr int kColMask = 0x7fffffff;
 constexpr int kSameBlock = (int)0x80000000u;  // low.x: same block row as the entry before it
-constexpr int kBeforeShift = 27;              // low.y: entries of the same row and tile before it, over
-constexpr int kSlotMask = (1 << 27) - 1;      //        its slot in U
+// pairs: x = slot of U_gb | kSameTarget | a << 27, y = slot of U_ga | kSameSum | b << 27
+constexpr int kSlotMask = (1 << 26) - 1;
+constexpr unsigned kSameTarget = 1u << 26;    // same (a, b) as the pair before it
+constexpr unsigned kSameSum = 1u << 26;       // and the same update block
+constexpr int kPlaceShift = 27;
 
-// a level-1 block row: its rows, its rows' run of entries of U', the place of
-// its packed pivot triangles (two 16-byte loads)
+// a level-1 block row: its rows, its rows' run of entries of U', its first
+// pair, the place of its packed pivot triangles (two 16-byte loads)
 struct alignas(16) Tile {
     int I, fr, h, entries;
-    int slot, pad;
+    int slot, pair;
     long long pk_off;
 };
 static_assert(sizeof(Tile) == 32, "Tile is two 16-byte words");
@@ -102,7 +105,9 @@ struct Pattern {
     bool mirrored = false;
     // two_level, parts of d_two: the level-1 block rows; K's row offsets; the level-0 fine rows; the
     // columns of U's entries, row after row; the entries of U', level-1 row
-    // after level-1 row; K's own entries of the level-1 pivot tiles with their
+    // after level-1 row (column, slot in U); the products U_ga D_g U_gb of the
+    // tiles' updates left of the diagonal (a < b), tile by tile, those of an
+    // entry (a, b) together and in row order; K's own entries of the level-1 pivot tiles with their
     // offsets per tile; per fine row its first entry in U (level 0) or U'
     // (level 1); per level-0 position of lvl_rows the fine rows before it
     DeviceBuffer d_two;
@@ -110,6 +115,7 @@ struct Pattern {
               *two_slot = nullptr, *two_l0_scan = nullptr;
     const two::Tile* two_tiles = nullptr;
     const int2 *two_low = nullptr, *two_tail = nullptr;
+    const uint2* two_pairs = nullptr;
     long long device_bytes = 0;
 };
 

@@ -250,44 +250,137 @@ __device__ __forceinline__ void step_2x2(T* Tt, T* D, int row, int len, double p
     __syncwarp();
 }
 
+// One pivot at row p (a single swap-and-step of d_factor_pivot_factorize);
+// returns its order
+template <class T>
+__device__ __forceinline__ int pivot_step(T* Tt, int p, int len, int* is_piv, T* D, int* perm, int method,
+                                          double piv64)
+{
+    const bool use_piv = method != CULIPX_PIV_STATIC;
+    int order = 1, p0 = p, p1 = p + 1;
+    if (p < len - 1 && method == CULIPX_PIV_BK) select_bk(Tt, p, len, order, p0, p1);
+    else if (p < len - 1 && method == CULIPX_PIV_ROOK) select_rook(Tt, p, len, order, p0, p1);
+    else order = (p < len - 1 && !is_piv[p + 1]) ? 2 : 1;
+    // lane 0 decides for the warp; for finite tiles every lane already
+    // agrees, and the clamp keeps the pivot rows inside the tile whatever
+    // the values (non-finite input yields a non-finite factor, no stray
+    // swap)
+    order = shfl(order, 0);
+    p0 = shfl(p0, 0);
+    p1 = shfl(p1, 0);
+    if (p0 < p || p0 >= len || (order == 2 && (p1 <= p || p1 >= len))) {
+        order = 1;
+        p0 = p;
+    }
+    __syncwarp();
+    if (order == 1) {
+        if (use_piv && p != p0) pivot_swap(Tt, perm, p, p0, len);
+        step_1x1(Tt, D, p, len);
+        if (use_piv && lane_id() == 0) is_piv[p] = 1;
+    } else {
+        if (use_piv) {
+            if (p0 != p) pivot_swap(Tt, perm, p, p0, len);
+            pivot_swap(Tt, perm, p + 1, p1, len);
+        }
+        step_2x2(Tt, D, p, len, piv64);
+        if (use_piv && lane_id() == 0) { is_piv[p] = 1; is_piv[p + 1] = 0; }
+    }
+    __syncwarp();
+    return order;
+}
+
 template <class T>
 __device__ __forceinline__ void factorize_tile(T* Tt, int len, int* is_piv, T* D, int* perm, int method,
                                                double piv64)
 {
-    const bool use_piv = method != CULIPX_PIV_STATIC;
-    int p = 0;
-    while (p < len) {
-        int order = 1, p0 = p, p1 = p + 1;
-        if (p < len - 1 && method == CULIPX_PIV_BK) select_bk(Tt, p, len, order, p0, p1);
-        else if (p < len - 1 && method == CULIPX_PIV_ROOK) select_rook(Tt, p, len, order, p0, p1);
-        else order = (p < len - 1 && !is_piv[p + 1]) ? 2 : 1;
-        // lane 0 decides for the warp; for finite tiles every lane already
-        // agrees, and the clamp keeps the pivot rows inside the tile whatever
-        // the values (non-finite input yields a non-finite factor, no stray
-        // swap)
-        order = shfl(order, 0);
-        p0 = shfl(p0, 0);
-        p1 = shfl(p1, 0);
-        if (p0 < p || p0 >= len || (order == 2 && (p1 <= p || p1 >= len))) {
-            order = 1;
-            p0 = p;
-        }
-        __syncwarp();
-        if (order == 1) {
-            if (use_piv && p != p0) pivot_swap(Tt, perm, p, p0, len);
-            step_1x1(Tt, D, p, len);
-            if (use_piv && lane_id() == 0) is_piv[p] = 1;
-        } else {
-            if (use_piv) {
-                if (p0 != p) pivot_swap(Tt, perm, p, p0, len);
-                pivot_swap(Tt, perm, p + 1, p1, len);
-            }
-            step_2x2(Tt, D, p, len, piv64);
-            if (use_piv && lane_id() == 0) { is_piv[p] = 1; is_piv[p + 1] = 0; }
-        }
-        __syncwarp();
-        p += order;
+    for (int p = 0; p < len;) p += pivot_step(Tt, p, len, is_piv, D, perm, method, piv64);
+}
+
+// factorize_tile for Bunch-Kaufman / Rook pivoting with the trailing rows in
+// registers: lane l holds column l of the next kWindow rows, t[0] being row p.
+// A step whose pivot stays in place (p passes both methods' first test, so the
+// step is a 1x1 without a swap) updates the window while it moves up by one
+// row, its multipliers broadcast from `row`; the rows below the window take
+// their updates when they enter it, in the same order.  Any other step brings
+// the tile up to date in shared memory and goes through pivot_step.  In shared
+// memory alone an update is a load, a shuffle and a store per row: 60 us of the
+// scale system's 111 (3125 tiles of 32, FP64).
+constexpr int kWindow = 16;
+constexpr int kRowBuf = 32 + kWindow;
+
+template <class T>
+__device__ __forceinline__ void pending_updates(T (&t)[kWindow], const T* Tt, int first, int k0, int k1, T pivots)
+{
+    const int l = lane_id();
+    for (int k = k0; k < k1; ++k) {
+        const T u = Tt[k * kTileStride + l], d = shfl(pivots, k);
+        const T* uk = Tt + k * kTileStride + first;
+#pragma unroll
+        for (int i = 0; i < kWindow; ++i)
+            if (first + i < 32) t[i] = fma_rn(-(uk[i] * d), u, t[i]);
     }
+}
+
+template <class T>
+__device__ __forceinline__ void factorize_tile_window(T* Tt, T* row, int len, int* is_piv, T* D, int* perm,
+                                                      int method, double piv64)
+{
+    const int l = lane_id();
+    const T alpha = bk_alpha<T>();
+    for (int e = l; e < kRowBuf; e += 32) row[e] = T(0);
+    __syncwarp();
+    T t[kWindow];
+    T pivots = T(0);  // lane k: the pivot of in-place step k
+    int p = 0, b0 = 0;  // the window was loaded at row b0
+    auto load = [&](int first) {
+#pragma unroll
+        for (int i = 0; i < kWindow; ++i) t[i] = (first + i < len) ? Tt[(first + i) * kTileStride + l] : T(0);
+    };
+    load(0);
+    while (p < len) {
+        T w = (l > p && l < len) ? fabs(t[0]) : T(0);
+        if (w != w) w = T(0);
+        const T w1 = max_bits(w);
+        T d11 = shfl(t[0], p);
+        if (p == len - 1 || !(w1 > T(0)) || fabs(d11) >= alpha * w1) {
+            // step_1x1 at p
+            const bool modified = fabs(d11) < 1e-8;
+            if (modified) d11 = T(1e-6);
+            const T u = ((l < p) ? T(0) : t[0]) / d11;
+            Tt[p * kTileStride + l] = (modified && l == p) ? T(1) : u;
+            row[l] = u * d11;
+            if (l == p) pivots = d11;
+            if (l < 3) D[3 * p + l] = (l != 1) ? T(0) : d11;
+            if (l == 0) is_piv[p] = 1;
+            __syncwarp();
+#pragma unroll
+            for (int i = 1; i < kWindow; ++i) t[i - 1] = fma_rn(-row[p + i], u, t[i]);
+            t[kWindow - 1] = T(0);
+            __syncwarp();
+            ++p;
+            if (p == b0 + kWindow && p < len) {
+                load(p);
+                pending_updates(t, Tt, p, b0, p, pivots);
+                b0 = p;
+            }
+            continue;
+        }
+#pragma unroll
+        for (int i = 0; i < kWindow; ++i)
+            if (p + i < b0 + kWindow && p + i < len) Tt[(p + i) * kTileStride + l] = t[i];
+        if (p > b0 && b0 + kWindow < len) {
+            load(b0 + kWindow);
+            pending_updates(t, Tt, b0 + kWindow, b0, p, pivots);
+#pragma unroll
+            for (int i = 0; i < kWindow; ++i)
+                if (b0 + kWindow + i < len) Tt[(b0 + kWindow + i) * kTileStride + l] = t[i];
+        }
+        __syncwarp();
+        p += pivot_step(Tt, p, len, is_piv, D, perm, method, piv64);
+        b0 = p;
+        load(p);
+    }
+    __syncwarp();
 }
 
 // ------------------------------- kernels ----------------------------------

@@ -125,7 +125,8 @@ void coarse_pattern(Pattern& p, const int* rowptr, const int* colidx)
 struct TwoLevel {
     std::vector<int> l0_rows, l0_scan, slot, ucol, tail_off;
     std::vector<int2> low, tail;
-    std::vector<two::Tile> tiles;
+    std::vector<uint2> pairs;
+    std::vector<two::Tile> tiles;  // one more than there are, for the last one's end
 };
 
 // Fills the two-level form; false where the pattern has none: other than two
@@ -172,6 +173,7 @@ bool two_level_form(Pattern& p, const int* rowptr, const int* colidx, TwoLevel& 
         two::Tile tile = {I, fr, blk_size(p, I), lower - w.slot[fr], w.slot[fr], 0, p.pk_off[I]};
         w.tiles.push_back(tile);
     }
+    w.tiles.push_back({0, 0, 0, 0, lower, 0, 0});
     if (entries != lower || entries == 0) return false;
     p.two_entries = entries;
     w.ucol.resize(entries);
@@ -198,13 +200,17 @@ bool two_level_form(Pattern& p, const int* rowptr, const int* colidx, TwoLevel& 
             }
         }
     }
+    // the entries of U' and the pairs, tile by tile: first counted, then placed
     bool ok = true;
+    std::vector<int> before(entries);
+    std::vector<long long> pair_off(q2 - q1 + 1, 0);
 #pragma omp parallel for schedule(static) reduction(&& : ok)
     for (int t = q1; t < q2; ++t) {
         const int I = p.lvl_rows[t], fr = p.bs[I];
+        long long pairs = 0;
         for (int i = fr; i < p.bs[I + 1]; ++i) {
-            int2* out = w.low.data() + w.slot[i];
-            for (int k = rowptr[i]; k < rowptr[i + 1] && colidx[k] < fr; ++k) {
+            int o = w.slot[i];
+            for (int k = rowptr[i]; k < rowptr[i + 1] && colidx[k] < fr; ++k, ++o) {
                 const int g = colidx[k];
                 const int* r0 = colidx + rowptr[g];
                 const int* r1 = colidx + rowptr[g + 1];
@@ -213,11 +219,52 @@ bool two_level_form(Pattern& p, const int* rowptr, const int* colidx, TwoLevel& 
                     ok = false;
                     break;
                 }
-                int before = 0;
-                while (at - before > r0 && at[-before - 1] >= fr) ++before;
-                const int slot = w.slot[g] + (int)(at - r0) - (r0[0] == g);
+                int n = 0;
+                while (at - n > r0 && at[-n - 1] >= fr) ++n;
+                before[o] = n;
+                pairs += n;
                 const bool same = k > rowptr[i] && p.row_block[g] == p.row_block[colidx[k - 1]];
-                *out++ = make_int2(g | (same ? two::kSameBlock : 0), (before << two::kBeforeShift) | slot);
+                w.low[o] = make_int2(g | (same ? two::kSameBlock : 0), w.slot[g] + (int)(at - r0) - (r0[0] == g));
+            }
+        }
+        pair_off[t - q1 + 1] = pairs;
+    }
+    if (!ok) return false;
+    for (int t = 0; t < q2 - q1; ++t) pair_off[t + 1] += pair_off[t];
+    // dense tiles (16 pairs an entry in full ones of 32) would take more memory
+    // than their blocks do; the general path stores those dense
+    if (pair_off[q2 - q1] > std::min(0x7fffffffLL, 8LL * entries + 4096)) return false;
+    w.pairs.resize((size_t)pair_off[q2 - q1]);
+    for (int t = 0; t <= q2 - q1; ++t) w.tiles[t].pair = (int)pair_off[t];
+#pragma omp parallel
+    {
+        struct Item {
+            int place, block, b, a;
+        };
+        std::vector<Item> items;
+#pragma omp for schedule(static)
+        for (int t = q1; t < q2; ++t) {
+            const int I = p.lvl_rows[t], fr = p.bs[I];
+            items.clear();
+            for (int i = fr; i < p.bs[I + 1]; ++i)
+                for (int k = rowptr[i], o = w.slot[i]; k < rowptr[i + 1] && colidx[k] < fr; ++k, ++o)
+                    for (int n = 1; n <= before[o]; ++n) {
+                        const int sb = w.low[o].y;
+                        items.push_back({(w.ucol[sb - n] & two::kColMask) - fr + 32 * (i - fr),
+                                         p.row_block[colidx[k]], sb, sb - n});
+                    }
+            // entry by entry; a stable sort keeps an entry's rows in order
+            std::stable_sort(items.begin(), items.end(),
+                             [](const Item& x, const Item& y) { return x.place < y.place; });
+            uint2* out = w.pairs.data() + pair_off[t - q1];
+            for (size_t k = 0; k < items.size(); ++k) {
+                const Item& m = items[k];
+                const bool target = k > 0 && items[k - 1].place == m.place;
+                const bool sum = target && items[k - 1].block == m.block;
+                *out++ = make_uint2((unsigned)m.b | (target ? two::kSameTarget : 0u) |
+                                        ((unsigned)(m.place & 31) << two::kPlaceShift),
+                                    (unsigned)m.a | (sum ? two::kSameSum : 0u) |
+                                        ((unsigned)(m.place >> 5) << two::kPlaceShift));
             }
         }
     }
@@ -472,7 +519,8 @@ int analyze_pattern(culipx_handle_t* h, int n, const int* rowptr, const int* col
             {form.tail_off.data(), sizeof(int) * form.tail_off.size()},
             {form.slot.data(), sizeof(int) * n},
             {form.l0_scan.data(), sizeof(int) * form.l0_scan.size()},
-            {form.tiles.data(), sizeof(two::Tile) * form.tiles.size()}};
+            {form.tiles.data(), sizeof(two::Tile) * form.tiles.size()},
+            {form.pairs.data(), sizeof(uint2) * form.pairs.size()}};
         size_t total = 0;
         for (const auto& q : parts) total += (q.second + 15) / 16 * 16;
         std::vector<unsigned char> all(total);
@@ -494,6 +542,7 @@ int analyze_pattern(culipx_handle_t* h, int n, const int* rowptr, const int* col
         p.two_slot = reinterpret_cast<const int*>(d + at[6]);
         p.two_l0_scan = reinterpret_cast<const int*>(d + at[7]);
         p.two_tiles = reinterpret_cast<const two::Tile*>(d + at[8]);
+        p.two_pairs = reinterpret_cast<const uint2*>(d + at[9]);
     }
     if (st != CULIPX_OK) { delete pp; return st; }
     p.device_bytes += (long long)p.d_two.bytes();
