@@ -53,13 +53,13 @@ PArgs<TF> make_args(Csr* A, Factor* M, double* base, double* partials, const dou
     a.cplx = M->cplx.as<int>();
     a.citem = M->citem.as<CItem>();
     const size_t vn = (size_t)n * nr;
-    for (int i = 0; i < 2; ++i) {
-        a.v[i] = base + (size_t)i * vn;
-        a.p[i] = base + (size_t)(2 + i) * vn;
-    }
-    a.Av = base + (size_t)4 * vn;
-    a.ev = base + (size_t)5 * vn;
-    a.xt = base + (size_t)6 * vn;
+    // the vectors that a solve reads before it writes them stand last (zero_vectors)
+    a.v[0] = base;
+    a.Av = base + vn;
+    a.ev = base + 2 * vn;
+    a.v[1] = base + 3 * vn;
+    for (int i = 0; i < 2; ++i) a.p[i] = base + (size_t)(4 + i) * vn;
+    a.xt = base + 6 * vn;
     a.out = base + (size_t)kVecs * vn;
     a.partials = partials;
     a.ts = nullptr;
@@ -128,14 +128,21 @@ int cached_grid(DeviceGridCache& c, SizeFn size, int* G, int* dev_out = nullptr)
     return CULIPX_OK;
 }
 
+// v_-1, p_-1, p_-2 and the iterate start at zero; everything else is written
+// before it is read, the caller's x among it
+template <class TF>
+int zero_vectors(const PArgs<TF>& a, int nr, cudaStream_t s)
+{
+    CULIPX_CUDA(cudaMemsetAsync(a.v[1], 0, (size_t)4 * a.n * nr * sizeof(double), s));
+    return CULIPX_OK;
+}
+
 // launch and wait; out_host receives 8 values per right-hand side
 template <class TF, int NR>
 int run_persistent(culipx_handle_t* h, PArgs<TF>& a, int G, double* out_host, bool wait = true)
 {
     cudaStream_t s = h->stream;
-    // the recurrence vectors start at zero; x is zeroed as in the reference
-    CULIPX_CUDA(cudaMemsetAsync(a.v[0], 0, (size_t)kVecs * a.n * NR * sizeof(double), s));
-    CULIPX_CUDA(cudaMemsetAsync(a.x, 0, (size_t)a.n * NR * sizeof(double), s));
+    CULIPX_TRY(zero_vectors(a, NR, s));
     void* args[] = {&a};
     CULIPX_CUDA(cudaLaunchCooperativeKernel(persistent_kernel<TF, NR>(), dim3(G), dim3(kT), args,
                                             res_smem_bytes<TF>(), s));
@@ -339,8 +346,7 @@ int launch_batched(Batch* bt, Csr* A, Factor* M, const double* b, double* x, dou
     ba.qe = bt->d_qe.as<int>();
     ba.out = bt->d_out.as<double>();
     ba.next = bt->d_next.as<int>();
-    CULIPX_CUDA(cudaMemsetAsync(a.v[0], 0, (size_t)kVecs * n * sizeof(double), s));
-    CULIPX_CUDA(cudaMemsetAsync(x, 0, (size_t)n * sizeof(double), s));
+    CULIPX_TRY(zero_vectors(a, 1, s));
     // static pivots or a threshold leave a factor whose level 0 is not known to be simple
     if (bt->lock.use && M->two_level && a.fuse_l0) return launch_lockstep<TF>(bt, a, w);
     CULIPX_CUDA(cudaMemsetAsync(ba.next, 0, sizeof(int), s));
