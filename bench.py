@@ -442,7 +442,7 @@ def sweep_roofline(F, N, flush, stream, reps=10, precision_bytes=8):
         out[name] = {"achieved": byt / (t * 1e-3) / 1e9, "frac": byt / (t * 1e-3) / 1e9 / peak,
                      "avg_us": t * 1e3, "algorithmic_bytes": int(byt)}
     out.update({"unit": "GB/s", "peak": peak, "peak_source": "MEASURED_PEAKS.json hbm_gbs (of measured)",
-                "kernels": "k_sweep_level per level (permutation folded in)",
+                "kernels": "k_two_left; k_two_right_tiles + k_two_right_rows (permutation folded in)",
                 "l2": "flushed before every call"})
     return out
 

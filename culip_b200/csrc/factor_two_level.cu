@@ -11,9 +11,8 @@
 // block by block and then re-lays U out as fine rows.  Here K's rows are read
 // as they are and the fine rows are written at once, in three launches:
 //   k_two_rows    thread per level-0 row: D and the row of U
-//   k_two_tiles   warp per level-1 block row: the Schur update (a lane per
-//                 tile column), the tile's factorization, its packed triangles
-//                 and its rows of U'
+//   k_two_tiles   warp per level-1 block row: the Schur update, the tile's
+//                 factorization, its packed triangles and its rows of U'
 //   k_two_order   the rows of U into the order of the permuted columns; the
 //                 level-1 block rows split into simple ones and work items
 // Every value and every order of summation is the general path's: an update
@@ -21,12 +20,12 @@
 // subtracted, blocks in row order; entries of sparse blocks with |u| <= NZ_EPS
 // are dropped.
 //
-// Bound: the tiles' serial pivot steps and the dependent loads of the Schur
-// lists, not bandwidth.  Measured on the scale system (n = 200 000,
-// m = 100 000, 3125 tiles of 32, FP64): 147 us (rows 13, tiles 111, order 22)
-// against 960 us for the general path's 31 launches, 590 of them in the
-// tiles' block-by-block updates; N = 3000 with tiles of 4: 21 us against 130;
-// 256 systems of 2.0 M rows in FP32: 0.57 ms against 3.4.
+// Bound: the tiles' serial pivot steps (short scoreboard and fixed latency, an
+// issue slot in three used), not bandwidth.  Measured on the scale system
+// (n = 200 000, m = 100 000, 3125 tiles of 32, FP64): 120 us (rows 13, tiles
+// 85, order 22) against 960 us for the general path's 31 launches, 590 of them
+// in the tiles' block-by-block updates; N = 3000 with tiles of 4: 18 us against
+// 130; 256 systems of 2.0 M rows in FP32: 0.46 ms against 3.4.
 #include "factor.h"
 #include "kernels_common.cuh"
 #include "launch.cuh"

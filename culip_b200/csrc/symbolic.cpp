@@ -134,8 +134,8 @@ struct TwoLevel {
 // pattern (the general path reads the upper triangle only and takes any), or
 // rows too long for a lane.  A lane walks a level-1 row and a thread a level-0
 // row, while the general path gives a tile's update blocks to a warp one by
-// one: about 1.4 us for each, measured, against 0.4 us here for each entry of a
-// tile's longest row.
+// one: about 1.4 us for each, measured, against at most 0.4 us here for each
+// entry of a tile's longest row.
 bool two_level_form(Pattern& p, const int* rowptr, const int* colidx, TwoLevel& w)
 {
     if (p.num_levels != 2 || !p.l0_diagonal || p.n > two::kRowMask || p.nnz > two::kSlotMask) return false;

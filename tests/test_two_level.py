@@ -56,6 +56,12 @@ def _system(form):
         A = _random_a(n, m, 0.02, rng)
         A[:, 3] = rng.standard_normal(m)
         A[5] = rng.standard_normal(n)
+    elif form == "wide":  # a tile's run of U' beyond what is staged at once, over several chunks
+        n, m, block = 900, 40, 32
+        A = _random_a(n, m, 0.05, rng)
+    elif form == "full32":  # full tiles of 32: more pairs than the two-level form takes
+        n, m, block = 96, 64, 32
+        A = _random_a(n, m, 1.0, rng)
     elif form == "tiny":  # pivots below the perturbation bound
         A = _random_a(n, m, 0.05, rng)
         h = rng.uniform(0.1, 10.0, n)
@@ -102,7 +108,7 @@ def _same_applies(F, OF, n, dtype):
 
 
 FORMS = ["block1", "block2", "block7", "block31", "block32", "dense", "mixed", "dropped", "long", "tiny", "swaps",
-         "nodiag", "lower", "unsymmetric"]
+         "wide", "full32", "nodiag", "lower", "unsymmetric"]
 
 
 @pytest.mark.parametrize("prec", [cb.F64, cb.F32])
