@@ -18,6 +18,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <new>
 #include <numeric>
 
 #include <omp.h>
@@ -236,6 +237,7 @@ bool two_level_form(Pattern& p, const int* rowptr, const int* colidx, TwoLevel& 
     if (pair_off[q2 - q1] > std::min(0x7fffffffLL, 8LL * entries + 4096)) return false;
     w.pairs.resize((size_t)pair_off[q2 - q1]);
     for (int t = 0; t <= q2 - q1; ++t) w.tiles[t].pair = (int)pair_off[t];
+    int no_memory = 0;
 #pragma omp parallel
     {
         struct Item {
@@ -246,6 +248,13 @@ bool two_level_form(Pattern& p, const int* rowptr, const int* colidx, TwoLevel& 
         for (int t = q1; t < q2; ++t) {
             const int I = p.lvl_rows[t], fr = p.bs[I];
             items.clear();
+            try {  // no exception may leave the parallel region
+                items.reserve((size_t)(pair_off[t - q1 + 1] - pair_off[t - q1]));
+            } catch (const std::bad_alloc&) {
+#pragma omp atomic write
+                no_memory = 1;
+                continue;
+            }
             for (int i = fr; i < p.bs[I + 1]; ++i)
                 for (int k = rowptr[i], o = w.slot[i]; k < rowptr[i + 1] && colidx[k] < fr; ++k, ++o)
                     for (int n = 1; n <= before[o]; ++n) {
@@ -268,6 +277,7 @@ bool two_level_form(Pattern& p, const int* rowptr, const int* colidx, TwoLevel& 
             }
         }
     }
+    if (no_memory) throw std::bad_alloc();
     return ok;
 }
 
