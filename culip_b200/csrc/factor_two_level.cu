@@ -104,7 +104,7 @@ template <class T>
 __device__ __forceinline__ T level0_pivot(const TwoArgs<T>& a, int tagged, int k0)
 {
     T d = T(0);
-    if (!(tagged & two::kNoDiag)) d = __ldg(a.kval + k0);
+    if (!(tagged & two::kNoDiag)) d = a.kval[k0];
     if (fabs(d) < 1e-8) d = T(1e-6);
     return d;
 }
@@ -137,7 +137,7 @@ __global__ void __launch_bounds__(256) k_two_rows(TwoArgs<T> a)
     for (int k = kb; k < k1; k += kRowRegs) {
         T v[kRowRegs];
 #pragma unroll
-        for (int j = 0; j < kRowRegs; ++j) v[j] = (k + j < k1) ? __ldg(a.kval + k + j) : T(0);
+        for (int j = 0; j < kRowRegs; ++j) v[j] = (k + j < k1) ? a.kval[k + j] : T(0);
 #pragma unroll
         for (int j = 0; j < kRowRegs; ++j) {
             if (k + j >= k1) break;
@@ -203,6 +203,7 @@ __global__ void __launch_bounds__(32 * kTileWarps, 6) k_two_tiles(TwoArgs<T> a)
     const int e0 = d1.x, e1 = d1.x + d0.w;
     int ut = k1;
     bool dropped = false;
+    // K's values were complete before the rows' kernel let this one start
     const int q0 = __ldg(a.tail_off + t), q1 = __ldg(a.tail_off + t + 1);
     row_s[warp][b] = T(0);
     __syncwarp();
@@ -369,7 +370,7 @@ __device__ void split_rows(const TwoArgs<T>& a, int q0)
     int s = 0, c = 0;  // simple rows and work items of this thread's share of the tiles before q0
     const uint4* kinds = reinterpret_cast<const uint4*>(a.kind);
     for (int i = tid; i < q0 / 16; i += kOrderT) {
-        const uint4 v = __ldg(kinds + i);
+        const uint4 v = kinds[i];
         const unsigned words[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -471,7 +472,7 @@ __global__ void __launch_bounds__(kOrderT) k_two_order(TwoArgs<T> a, int splits)
 #pragma unroll
         for (int j = 0; j < kRowRegs; ++j) {
             const bool keep = v[j] != T(0);
-            nc[j] = keep ? __ldg(a.iperm + c[j]) : two::kColMask;
+            nc[j] = keep ? a.iperm[c[j]] : two::kColMask;
             kept += keep;
         }
 #pragma unroll
@@ -493,7 +494,7 @@ __global__ void __launch_bounds__(kOrderT) k_two_order(TwoArgs<T> a, int splits)
     for (int j = 0; j < len; ++j) {  // insertion: an entry moves within its block's few
         const T v = a.up[o0 + j].x;
         if (v == T(0)) continue;
-        const int c = __ldg(a.ucol + o0 + j) & two::kColMask, nc = __ldg(a.iperm + c);
+        const int c = __ldg(a.ucol + o0 + j) & two::kColMask, nc = a.iperm[c];
         int k = o++;
         for (; k > o0 && a.u_col[k - 1] > nc; --k) {
             a.u_col[k] = a.u_col[k - 1];

@@ -36,9 +36,8 @@ constexpr int kPerThread = 4;
 
 template <class TO>
 __global__ void __launch_bounds__(256) k_kkt_values(int nnz_k, int n, const int* __restrict__ src,
-                                                    const double* __restrict__ aval, const double* __restrict__ x,
-                                                    const double* __restrict__ s, const double* __restrict__ d,
-                                                    double delta, double gamma, TO* __restrict__ kval)
+                                                    const double* aval, const double* x, const double* s,
+                                                    const double* d, double delta, double gamma, TO* kval)
 {
     const long long e0 = (long long)blockIdx.x * (256 * kPerThread) + threadIdx.x;
     int q[kPerThread];
@@ -51,10 +50,10 @@ __global__ void __launch_bounds__(256) k_kkt_values(int nnz_k, int n, const int*
         v[j] = 0.0;
         if (e0 + 256 * j >= nnz_k) continue;
         if (q[j] >= 0) {
-            v[j] = __ldg(aval + q[j]);
+            v[j] = aval[q[j]];
         } else {
             const int r = -1 - q[j];
-            if (r < n) v[j] = (d ? __ldg(d + r) : __ldg(s + r) / __ldg(x + r)) + delta;
+            if (r < n) v[j] = (d ? d[r] : s[r] / x[r]) + delta;
             else v[j] = -gamma;
         }
     }

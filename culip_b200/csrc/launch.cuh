@@ -8,6 +8,12 @@
 // part may read what was complete before its predecessor began: the successor
 // of a kernel that has passed after_previous starts after everything before
 // that kernel is complete and visible.
+//
+// Such a kernel's life begins before its predecessor has finished writing, so
+// what the predecessor may write is read with plain loads through pointers
+// without __restrict__: __ldg and const __restrict__ promise that nothing
+// writes the memory during the kernel's life, and leave the compiler free to
+// move the load above after_previous().
 #pragma once
 
 #include "device.h"

@@ -30,10 +30,12 @@ namespace culipx {
 
 namespace {
 
+// x, y and a CSR's values may be the output of the kernel before (launch.cuh);
+// a SELL copy's values are refreshed by an ordinary launch.
 template <class T, int L>
 __global__ void __launch_bounds__(256) k_csr_spmv(int m, const int* __restrict__ rowptr,
-                                                  const int* __restrict__ colidx, const T* __restrict__ val,
-                                                  const T* __restrict__ x, T* __restrict__ y, T alpha, T beta)
+                                                  const int* __restrict__ colidx, const T* val, const T* x, T* y,
+                                                  T alpha, T beta)
 {
     after_previous();
     constexpr int kRowsPerWarp = 32 / L;
@@ -47,7 +49,7 @@ __global__ void __launch_bounds__(256) k_csr_spmv(int m, const int* __restrict__
         if (row < m) {
             const int e = __ldg(rowptr + row + 1);
             for (int k = __ldg(rowptr + row) + sub; k < e; k += L)
-                acc = fma_rn(__ldg(val + k), __ldg(x + __ldg(colidx + k)), acc);
+                acc = fma_rn(val[k], x[__ldg(colidx + k)], acc);
         }
 #pragma unroll
         for (int o = L / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
@@ -62,8 +64,8 @@ constexpr int kGatherBatch = 8;
 
 template <class T>
 __global__ void __launch_bounds__(256) k_csr_spmv_rows(int m, const int* __restrict__ rowptr,
-                                                       const int* __restrict__ colidx, const T* __restrict__ val,
-                                                       const T* __restrict__ x, T* __restrict__ y, T alpha, T beta)
+                                                       const int* __restrict__ colidx, const T* val, const T* x, T* y,
+                                                       T alpha, T beta)
 {
     after_previous();
     const int row = blockIdx.x * blockDim.x + threadIdx.x;
@@ -83,10 +85,10 @@ __global__ void __launch_bounds__(256) k_csr_spmv_rows(int m, const int* __restr
             for (int j = 0; j < kGatherBatch; ++j) {
                 const bool ok = kb + j < re;
                 c[j] = ok ? __ldg(colidx + kb + j) : -1;
-                v[j] = ok ? __ldg(val + kb + j) : T(0);
+                v[j] = ok ? val[kb + j] : T(0);
             }
 #pragma unroll
-            for (int j = 0; j < kGatherBatch; ++j) xv[j] = (c[j] >= 0) ? __ldg(x + c[j]) : T(0);
+            for (int j = 0; j < kGatherBatch; ++j) xv[j] = (c[j] >= 0) ? x[c[j]] : T(0);
 #pragma unroll
             for (int j = 0; j < kGatherBatch; ++j)
                 if (c[j] >= 0) acc = fma_rn(v[j], xv[j], acc);
@@ -99,7 +101,7 @@ __global__ void __launch_bounds__(256) k_csr_spmv_rows(int m, const int* __restr
         todo &= todo - 1;
         const int a = __shfl_sync(0xffffffffu, rs, src), e = __shfl_sync(0xffffffffu, re, src);
         T part = T(0);
-        for (int k = a + lane; k < e; k += 32) part = fma_rn(__ldg(val + k), __ldg(x + __ldg(colidx + k)), part);
+        for (int k = a + lane; k < e; k += 32) part = fma_rn(val[k], x[__ldg(colidx + k)], part);
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
         if (lane == src) acc = part;
@@ -142,8 +144,7 @@ template <class T>
 __global__ void __launch_bounds__(128) k_sell_spmv(int nslices, const int* __restrict__ rows,
                                                    const long long* __restrict__ slice_off,
                                                    const int* __restrict__ slice_len, const int* __restrict__ col,
-                                                   const T* __restrict__ val, const T* __restrict__ x,
-                                                   T* __restrict__ y, T alpha, T beta)
+                                                   const T* __restrict__ val, const T* x, T* y, T alpha, T beta)
 {
     after_previous();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -166,7 +167,7 @@ __global__ void __launch_bounds__(128) k_sell_spmv(int nslices, const int* __res
     for (int jb = 0; jb < len; jb += B) {
         T xv[B];
 #pragma unroll
-        for (int j = 0; j < B; ++j) xv[j] = (c[j] >= 0) ? __ldg(x + c[j]) : T(0);
+        for (int j = 0; j < B; ++j) xv[j] = (c[j] >= 0) ? x[c[j]] : T(0);
         // the next batch's indices and values, in flight with this batch's gathers
         int cn[B];
         T vn[B];
@@ -193,8 +194,7 @@ __global__ void __launch_bounds__(128) k_sell_spmv(int nslices, const int* __res
 template <class T>
 __global__ void __launch_bounds__(256) k_long_rows(int nlong, const int* __restrict__ list,
                                                    const long long* __restrict__ off, const int* __restrict__ col,
-                                                   const T* __restrict__ val, const T* __restrict__ x,
-                                                   T* __restrict__ y, T alpha, T beta)
+                                                   const T* __restrict__ val, const T* x, T* y, T alpha, T beta)
 {
     after_previous();
     const int lane = lane_id();
@@ -203,7 +203,7 @@ __global__ void __launch_bounds__(256) k_long_rows(int nlong, const int* __restr
         const int row = __ldg(list + w);
         const long long a = __ldg(off + w), e = __ldg(off + w + 1);
         T part = T(0);
-        for (long long k = a + lane; k < e; k += 32) part = fma_rn(__ldg(val + k), __ldg(x + __ldg(col + k)), part);
+        for (long long k = a + lane; k < e; k += 32) part = fma_rn(__ldg(val + k), x[__ldg(col + k)], part);
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
         if (lane == 0) y[row] = (beta == T(0)) ? alpha * part : fma_rn(alpha, part, beta * y[row]);
