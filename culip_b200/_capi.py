@@ -128,6 +128,7 @@ _SIGS = {
                            ctypes.POINTER(i32)],
     "culipx_sqmr_profile": [vp, i32],
     "culipx_sqmr_set_wait_skew": [vp, ctypes.c_ulonglong],
+    "culipx_sqmr_set_reduce_skew": [vp, ctypes.c_ulonglong],
     "culipx_sqmr_phase_times": [vp, vp, i32],
 }
 

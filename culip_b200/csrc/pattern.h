@@ -71,6 +71,7 @@ struct Pattern {
     // between two rows of the same level-0 block row): a level-0 row's K row
     // then reads only itself and rows of later levels
     bool l0_diagonal = false;
+    int longest_row = 0;         // entries of K's longest row
     // two levels whose level-0 block rows have diagonal pivot blocks, rows of
     // moderate length (a KKT system in its natural order at fill level 0): the
     // factor runs on K's fine rows (factor_two_level.cu).  The device arrays

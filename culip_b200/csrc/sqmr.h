@@ -17,6 +17,7 @@ struct Sqmr {
     bool force_multi_kernel = false;  // use the per-phase kernels instead of the persistent solver
     bool profile = false;             // record per-phase device timestamps of the persistent solver
     unsigned long long wait_skew = 0; // added to the persistent solver's level-wait target (tests; 0)
+    unsigned long long red_skew = 0;  // the same for its reductions' counted barrier
     DeviceBuffer ts;                  // 64 iterations x 8 phase stamps (ns, %globaltimer)
     DeviceBuffer vecs, partials, scal;
     DeviceBuffer ref_r, ref_d, ref_part;  // iterative refinement: residual, correction, norm partials

@@ -65,9 +65,29 @@ PArgs<TF> make_args(Csr* A, Factor* M, double* base, double* partials, const dou
     a.ts = nullptr;
     a.lvl_done = nullptr;
     a.wait_skew = 0;
+    a.count_red = 0;
+    a.red_skew = 0;
     a.x = x;
     a.b = b;
     return a;
+}
+
+// Whether the reductions of a fused two-level solve on G CTAs may use the
+// counted barrier, whose wait is bounded (kWaitLimitNs, 200 ms).  They wait
+// for the slowest thread of a phase; a thread walks a row of K and its run of
+// U' serially.  At most kCountedSerial entries to a thread, each at most twice
+// in a phase and each walk at most 1 us an entry (two dependent trips to
+// memory for two entries with four right-hand sides), is 33 ms.  Longer rows
+// (a dense constraint, say) keep grid.sync, which waits as long as they take:
+// next to such a phase the 0.5 us that the counted barrier saves are nothing.
+constexpr long long kCountedSerial = 16384;
+
+bool reductions_counted(const Pattern& p, int G)
+{
+    if (p.num_levels != 2) return false;
+    const long long items = p.lvl_off[2] - p.lvl_off[1];
+    const long long rows = items / ((long long)G * kW) + p.n / ((long long)G * kT) + 2;  // of one thread
+    return rows * p.longest_row <= kCountedSerial;
 }
 
 int ctas_per_sm()
@@ -172,6 +192,8 @@ int launch_persistent(culipx_handle_t* h, Csr* A, Factor* M, const double* b, do
     // the level counter in the spare slots after the results (need: 8 NR + 64 values)
     a.lvl_done = reinterpret_cast<unsigned long long*>(a.out + 8 * kMaxNR);
     a.wait_skew = w->wait_skew;
+    a.count_red = reductions_counted(*M->pat, G);
+    a.red_skew = w->red_skew;
     if (w->profile && NR == 1) {
         if (w->ts.bytes() < (size_t)kTsIters * 8 * sizeof(unsigned long long))
             CULIPX_TRY(w->ts.alloc(h, (size_t)kTsIters * 8 * sizeof(unsigned long long)));
@@ -838,6 +860,8 @@ int launch_noalloc(culipx_handle_t* h, Csr* A, Factor* M, const double* b, doubl
     // the level counter after the results (the vectors' region holds a spare row of kNoAllocMaxRows values)
     a.lvl_done = reinterpret_cast<unsigned long long*>(a.out + 8 * kMaxNR);
     a.wait_skew = h->sqmr ? h->sqmr->wait_skew : 0;
+    a.count_red = reductions_counted(*M->pat, G);
+    a.red_skew = h->sqmr ? h->sqmr->red_skew : 0;
     return run_persistent<TF, 1>(h, a, G, out);
 }
 

@@ -32,9 +32,11 @@
 // level-0 phase goes away), and instead of a grid barrier between the U
 // sweep's two levels every CTA counts its finished level-1 rows on a device
 // counter that the level-0 rows wait for (one elected poller per CTA, a
-// bounded wait: a wait that gives up ends the solve with CULIPX_TIMEOUT) --
-// two grid synchronisations per iteration, both reductions.  Re-associations against the reference, all exact in
-// real arithmetic:
+// bounded wait: a wait that gives up ends the solve with CULIPX_TIMEOUT).
+// The two reductions are then the iteration's only grid-wide barriers, and
+// where every phase is short they are counted and bounded the same way
+// (grid_reduce).  Re-associations against the reference, all exact in real
+// arithmetic:
 //   * v+ is divided by delta after the U sweep instead of before it (the
 //     sweep is linear); the division is applied to the SpMV result.
 //   * The reference's w_k (sqmr.impl.cuh, solve_middle of v_k scaled by eta
@@ -83,6 +85,7 @@ template <class TF>
 struct PArgs {
     int n, nl, max_it;
     int fuse_l0;               // level-0 simple rows compute (K ev) in the U sweep
+    int count_red;             // the fused iteration's reductions may use the counted barrier
     double tol;
     const int* rowptr;
     const int* colidx;
@@ -126,10 +129,13 @@ struct PArgs {
     // G (it + 1) before they read them.  [1]: set when a wait gave up.
     unsigned long long* lvl_done;  // [2], [3]: the same for the reductions' barrier
     unsigned long long wait_skew;  // added to the wait's target (fault injection in tests; 0)
+    unsigned long long red_skew;   // the same for the reductions' counted barrier
 };
 
-// Bound of one device wait on the level counter: well above any legitimate
-// wait (a few microseconds), far below a watchdog.
+// Bound of one device wait on a counter, far below a watchdog.  The level
+// handoff waits for level-1 tiles, which walk no rows: a few microseconds.
+// The reductions wait for whole phases and are counted only where the rows
+// keep those well under it (reductions_counted, sqmr_persistent.cu).
 constexpr unsigned long long kWaitLimitNs = 200ull * 1000 * 1000;
 
 // Shared state of a CTA's level waits: the iteration (+1) whose count the CTA
@@ -206,12 +212,20 @@ __host__ __device__ __forceinline__ int acc3(int r) { return (r % 3) + ((r < 0) 
 // 0 derives from them with a __syncthreads() before the next reduction.
 // ctr (counter, gave-up flag): the barrier is one release add per CTA and one
 // acquiring poller, a round trip to L2 less than grid.sync's (scale: 1656 ->
-// 1621 us for 32 iterations); the wait is bounded (wait_count), and a wait that
-// gives up lets every later one pass.  NULL: grid.sync.
+// 1621 us for 32 iterations); the wait is bounded (wait_count).  NULL:
+// grid.sync.
+// Thread 0 gets false when its wait gave up: the totals are then not the
+// grid's and may differ between CTAs, so the caller must leave its loop, and
+// that loop may hold no grid.sync of its own (the CTAs need not leave at the
+// same iteration).  They all leave soon: the first CTA that gave up adds at
+// most one more count (the iteration's second reduction), so no later target
+// is reached, and with the flag set a wait short of its target gives up at
+// once.
 template <int NV>
-__device__ void grid_reduce(double (&v)[NV], double* partials, int& red, double (*sh)[kW], cg::grid_group& grid,
-                            unsigned long long* ctr, int counted_from)
+__device__ bool grid_reduce(double (&v)[NV], double* partials, int& red, double (*sh)[kW], cg::grid_group& grid,
+                            unsigned long long* ctr, int counted_from, unsigned long long skew)
 {
+    bool ok = true;
     const int lane = (int)lane_id(), w = threadIdx.x >> 5;
 #pragma unroll
     for (int k = 0; k < NV; ++k)
@@ -232,10 +246,11 @@ __device__ void grid_reduce(double (&v)[NV], double* partials, int& red, double 
             __syncwarp();
             if (lane == 0) {
                 red_release_add_u64(ctr, 1ull);
-                const unsigned long long target = (unsigned long long)gridDim.x * (unsigned long long)(red - counted_from);
+                const unsigned long long target =
+                    (unsigned long long)gridDim.x * (unsigned long long)(red - counted_from) + skew;
                 int k = 0;
                 while (k < 64 && ld_acquire_u64(ctr) < target) ++k;  // the others are usually close behind
-                if (k == 64) wait_count(ctr, target);
+                if (k == 64) ok = wait_count(ctr, target);
             }
         }
         __syncthreads();
@@ -263,6 +278,7 @@ __device__ void grid_reduce(double (&v)[NV], double* partials, int& red, double 
             for (int i = 0; i < kW; ++i) t += sh[k][i];
             v[k] = t;
         }
+    return ok;
 }
 
 // D^-1 of one block row (k_solve_D, helper_kernels.impl.cuh:720-774).  With
@@ -846,6 +862,19 @@ inline __device__ void scal_after_ut(Scal& Q, double vda, double wda, double wdw
     }
 }
 
+// A reduction's wait gave up: the solve ends here (its results are marked
+// invalid by the counter's flag)
+template <int NR>
+__device__ __forceinline__ void abandon(Scal (&S)[NR], int it)
+{
+    for (int j = 0; j < NR; ++j) {
+        if (S[j].done) continue;
+        S[j].done = 1;
+        S[j].iters = it;
+        S[j].stop_it = it;
+    }
+}
+
 // Fixed-order sum over one CTA: thread 0 gets the totals (same protocol as
 // grid_reduce).
 template <int NV>
@@ -878,30 +907,32 @@ struct GridCtx {
     int wid, nwarps, g0, gstride;
     unsigned long long* ctr;  // the reductions' barrier (grid_reduce); NULL before begin_counted
     int counted_from;         // reductions before it
+    unsigned long long skew;  // added to their targets (tests)
     __device__ void sync() { grid.sync(); }
     // from here on the reductions use the counter behind the level counter,
-    // zeroed before the initial phases
-    __device__ void begin_counted(unsigned long long* lvl_done)
+    // zeroed before the initial phases; only for a loop without sync()
+    __device__ void begin_counted(unsigned long long* lvl_done, unsigned long long red_skew)
     {
-        if (!lvl_done) return;
         ctr = lvl_done + 2;
         counted_from = red;  // red goes on: the partials' two buffers keep alternating
+        skew = red_skew;
     }
     template <int NV>
-    __device__ void reduce(double (&v)[NV], double (*sh)[kW])
+    __device__ bool reduce(double (&v)[NV], double (*sh)[kW])
     {
-        grid_reduce<NV>(v, partials, red, sh, grid, ctr, counted_from);
+        return grid_reduce<NV>(v, partials, red, sh, grid, ctr, counted_from, skew);
     }
 };
 
 struct CtaCtx {
     int wid, nwarps, g0, gstride;
     __device__ void sync() const { __syncthreads(); }
-    __device__ void begin_counted(unsigned long long*) const {}
+    __device__ void begin_counted(unsigned long long*, unsigned long long) const {}
     template <int NV>
-    __device__ void reduce(double (&v)[NV], double (*sh)[kW])
+    __device__ bool reduce(double (&v)[NV], double (*sh)[kW])
     {
         cta_reduce<NV>(v, sh);
+        return true;
     }
 };
 
@@ -1193,7 +1224,8 @@ __device__ void sqmr_body(const PArgs<TF>& a, Ctx& ctx, const SysView& sv, Scal 
         __syncthreads();
     }
 
-    ctx.begin_counted(a.lvl_done);
+    // the counted iteration has no ctx.sync() between here and the loop's end
+    if (counted && a.count_red) ctx.begin_counted(a.lvl_done, a.red_skew);
     int it = 0;
     for (;;) {
         bool any = false;
@@ -1301,7 +1333,8 @@ __device__ void sqmr_body(const PArgs<TF>& a, Ctx& ctx, const SysView& sv, Scal 
                     if (NR == 1 && L == a.nl - 1) stamp(a.ts, it, 1);
                 }
             }
-            ctx.template reduce<NR>(r, sh);
+            const bool ok = ctx.template reduce<NR>(r, sh);
+            if (tid == 0 && !ok) abandon<NR>(S, it);
             if (tid == 0)
                 for (int j = 0; j < NR; ++j) {
                     if (S[j].done) continue;
@@ -1467,7 +1500,8 @@ __device__ void sqmr_body(const PArgs<TF>& a, Ctx& ctx, const SysView& sv, Scal 
                     if (NR == 1 && L == 0) stamp(a.ts, it, 4);
                 }
             }
-            ctx.template reduce<4 * NR>(r, sh);
+            const bool ok = ctx.template reduce<4 * NR>(r, sh);
+            if (tid == 0 && !ok) abandon<NR>(S, it);
             if (tid == 0)
                 for (int j = 0; j < NR; ++j) {
                     if (S[j].done) continue;
@@ -1527,7 +1561,7 @@ __global__ void __launch_bounds__(kT, CTAS) k_sqmr_persistent(PArgs<TF> a)
     extern __shared__ __align__(16) unsigned char res_smem[];
     const int G = gridDim.x;
     GridCtx ctx{cg::this_grid(), a.partials, 0, (int)(threadIdx.x >> 5) * G + (int)blockIdx.x,  // items interleaved
-                G * kW, (int)(blockIdx.x * kT + threadIdx.x), G * kT, nullptr, 0};
+                G * kW, (int)(blockIdx.x * kT + threadIdx.x), G * kT, nullptr, 0, 0ull};
     const SysView sv{0, a.n, a.lvl_off, a.lvl_off + 1, blockIdx.x == 0 ? a.out : nullptr};
     sqmr_body<TF, NR>(a, ctx, sv, S, sh, reinterpret_cast<ResSlot<TF>*>(res_smem));
 }

@@ -340,6 +340,7 @@ int analyze_pattern(culipx_handle_t* h, int n, const int* rowptr, const int* col
             b0 = b1;
         }
     }
+    for (int i = 0; i < n; ++i) p.longest_row = std::max(p.longest_row, rowptr[i + 1] - rowptr[i]);
     for (int i = 0; i < n; ++i)
         for (int q = rowptr[i]; q < rowptr[i + 1]; ++q)
             if (colidx[q] < 0 || colidx[q] >= n || (q > rowptr[i] && colidx[q] <= colidx[q - 1])) {

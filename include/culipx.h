@@ -549,6 +549,10 @@ int culipx_sqmr_profile(culipx_handle h, int enable);
  * gives up and the solve returns CULIPX_TIMEOUT (results invalid) instead of
  * hanging.  0 (the default) for normal operation. */
 int culipx_sqmr_set_wait_skew(culipx_handle h, unsigned long long skew);
+/* The same for the iteration's grid-wide reductions, whose wait is bounded
+ * (200 ms) only for two-level systems with short rows; any other solve keeps
+ * an unbounded grid barrier there and ignores the skew. */
+int culipx_sqmr_set_reduce_skew(culipx_handle h, unsigned long long skew);
 int culipx_sqmr_phase_times(culipx_handle h, double *out_us, int iterations);
 
 /* The same solve (same kernel, same results) without any device allocation;
