@@ -57,6 +57,20 @@ unsigned long long next_serial();
 // Checks the last launch error on this thread.
 int launch_check(const char* what);
 
+// While it lives, this thread may allocate and copy although a stream (the
+// caller's own, or another thread's) is being captured; nothing of it is
+// captured.
+class OutsideCapture {
+public:
+    OutsideCapture() { cudaThreadExchangeStreamCaptureMode(&mode_); }
+    ~OutsideCapture() { cudaThreadExchangeStreamCaptureMode(&mode_); }
+    OutsideCapture(const OutsideCapture&) = delete;
+    OutsideCapture& operator=(const OutsideCapture&) = delete;
+
+private:
+    cudaStreamCaptureMode mode_ = cudaStreamCaptureModeRelaxed;
+};
+
 // Device memory charged against the owning handle's budget.
 class DeviceBuffer {
 public:

@@ -936,11 +936,14 @@ int run_levels(Factor* f, const void* d_vals, cudaStream_t s, int* launches)
 }  // namespace
 
 int build_sweeps(Factor* f, cudaStream_t stream, int* launches);  // solve.cu
+size_t exclusive_scan_bytes(int n);                               // solve.cu
 
 namespace {
 
 // The general path's block storage: with the factor for most patterns; for a
-// two-level one only once static pivots or a threshold call for it.
+// two-level one only once static pivots or a threshold call for it.  That call
+// may be the first that a caller captures (ordinary ones before it having run
+// on fine rows), so all that it allocates comes from here.
 int block_storage(Factor* f)
 {
     const Pattern& p = *f->pat;
@@ -959,7 +962,8 @@ int block_storage(Factor* f)
     al(f->state, 16 * sizeof(long long));
     al(f->deferred, (size_t)std::max(p.max_level_blocks, 1) * sizeof(int));
     al(f->slowlist, (size_t)std::max(p.max_level_blocks, 1) * sizeof(int));
-    al(f->piv_off, p.num_blocks * sizeof(long long));
+    if (p.two_level) al(f->scan_tmp, exclusive_scan_bytes(p.n + 1));
+    al(f->piv_off, p.num_blocks * sizeof(long long));  // the last one
     return st;
 }
 
@@ -1050,8 +1054,11 @@ int factor_compute(Factor* f, const void* d_vals, const int* h_is_piv, int pivot
         f->computed = true;
         return CULIPX_OK;
     }
-    CULIPX_TRY(block_mirror(p));
-    CULIPX_TRY(block_storage(f));
+    if (!f->piv_off.get()) {
+        OutsideCapture allocate;
+        CULIPX_TRY(block_mirror(p));
+        CULIPX_TRY(block_storage(f));
+    }
     CULIPX_CUDA(cudaMemsetAsync(f->val.get(), 0, p.val_slots * f->vbytes, s));
     CULIPX_CUDA(cudaMemcpyAsync(f->idx.get(), p.d_idx_init.get(), p.val_slots * sizeof(int),
                                 cudaMemcpyDeviceToDevice, s));

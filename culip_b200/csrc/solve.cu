@@ -813,10 +813,12 @@ int apply_t(Factor* f, int stage, const void* d_b, void* d_x, cudaStream_t s)
 
 // exclusive scan of n int counts in place (n - 1 counts and a trailing 0 give
 // the offsets and the total), three launches
+size_t exclusive_scan_bytes(int n) { return (size_t)((n + kScanChunk - 1) / kScanChunk) * sizeof(int); }
+
 int exclusive_scan(int* d, int n, DeviceBuffer& tmp, culipx_handle_t* h, cudaStream_t s, int* launches)
 {
     const int chunks = (n + kScanChunk - 1) / kScanChunk;
-    if ((size_t)chunks * sizeof(int) > tmp.bytes()) CULIPX_TRY(tmp.alloc(h, (size_t)chunks * sizeof(int)));
+    if (exclusive_scan_bytes(n) > tmp.bytes()) CULIPX_TRY(tmp.alloc(h, exclusive_scan_bytes(n)));
     k_scan_chunks<<<chunks, kScanThreads, 0, s>>>(d, n, tmp.as<int>());
     k_scan_sums<<<1, 1024, 0, s>>>(tmp.as<int>(), chunks);
     k_scan_add<<<chunks, kScanThreads, 0, s>>>(d, n, tmp.as<int>());

@@ -593,24 +593,44 @@ int block_mirror(Pattern& p)
             }
     }
 
+    // on a stream of its own: a copy on the legacy stream would end the
+    // capture of a blocking stream
+    const struct {
+        DeviceBuffer& buf;
+        const void* src;
+        size_t size;
+    } parts[] = {{p.d_cs_off, p.cs_off.data(), sizeof(int) * (cm + 1)},
+                 {p.d_row_offdiag_start, p.row_offdiag_start.data(), sizeof(int) * cm},
+                 {p.d_desc, p.desc.data(), sizeof(BlockDesc) * cnz},
+                 {p.d_csc_off, p.csc_off.data(), sizeof(int) * (cm + 1)},
+                 {p.d_csc_blk, p.csc_blk.data(), sizeof(int) * cnz},
+                 {p.d_lb, p.lb.data(), sizeof(int) * cnz},
+                 {p.d_a_dst, a_dst.data(), sizeof(int) * p.nnz},
+                 {p.d_idx_init, idx_init.data(), sizeof(int) * p.val_slots},
+                 {p.d_nnz_init, nnz_init.data(), sizeof(int) * cnz},
+                 {p.d_fmt, p.fmt.data(), sizeof(int) * cnz},
+                 {p.d_maxnnz, p.max_nnz.data(), sizeof(int) * cnz}};
+    cudaStream_t s = nullptr;
+    CULIPX_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+    int st = CULIPX_OK;
     long long bytes = 0;
-    auto up = [&](DeviceBuffer& buf, const void* src, size_t size) -> int {
-        if (buf.get()) return CULIPX_OK;  // an earlier call that ran out of memory got this far
-        CULIPX_TRY(buf.upload(h, src, size));
-        bytes += (long long)buf.bytes();
+    auto up = [&]() -> int {
+        for (const auto& q : parts) {
+            CULIPX_TRY(q.buf.alloc(h, q.size));
+            if (q.size) CULIPX_CUDA(cudaMemcpyAsync(q.buf.get(), q.src, q.size, cudaMemcpyHostToDevice, s));
+            bytes += (long long)q.buf.bytes();
+        }
         return CULIPX_OK;
     };
-    CULIPX_TRY(up(p.d_cs_off, p.cs_off.data(), sizeof(int) * (cm + 1)));
-    CULIPX_TRY(up(p.d_row_offdiag_start, p.row_offdiag_start.data(), sizeof(int) * cm));
-    CULIPX_TRY(up(p.d_desc, p.desc.data(), sizeof(BlockDesc) * cnz));
-    CULIPX_TRY(up(p.d_csc_off, p.csc_off.data(), sizeof(int) * (cm + 1)));
-    CULIPX_TRY(up(p.d_csc_blk, p.csc_blk.data(), sizeof(int) * cnz));
-    CULIPX_TRY(up(p.d_lb, p.lb.data(), sizeof(int) * cnz));
-    CULIPX_TRY(up(p.d_a_dst, a_dst.data(), sizeof(int) * p.nnz));
-    CULIPX_TRY(up(p.d_idx_init, idx_init.data(), sizeof(int) * p.val_slots));
-    CULIPX_TRY(up(p.d_nnz_init, nnz_init.data(), sizeof(int) * cnz));
-    CULIPX_TRY(up(p.d_fmt, p.fmt.data(), sizeof(int) * cnz));
-    CULIPX_TRY(up(p.d_maxnnz, p.max_nnz.data(), sizeof(int) * cnz));
+    st = up();
+    const cudaError_t e = cudaStreamSynchronize(s);
+    cudaStreamDestroy(s);
+    if (st == CULIPX_OK && e != cudaSuccess)
+        st = fail(CULIPX_CUDA_ERROR, "uploading the block form failed: %s", cudaGetErrorString(e));
+    if (st != CULIPX_OK) {  // the next call starts over
+        for (const auto& q : parts) q.buf.release();
+        return st;
+    }
     p.device_bytes += bytes;
     p.k_rowptr = std::vector<int>();
     p.k_colidx = std::vector<int>();
