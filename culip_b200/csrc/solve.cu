@@ -588,15 +588,26 @@ __global__ void __launch_bounds__(32 * kSweepWarps)
 
 // one block-Jacobi sweep over all block rows (SOLVE_JACOBI; the stripe
 // kernel of solve_U_jacobi / solve_Ut_jacobi, block_ildlt.impl.cuh:2455-2494
-// and 2635-2674): x_out_I = U_II^-1 (b_I - U_I* x_in) for U (UPPER) or U'
+// and 2635-2674): x_out_I = U_II^-1 (b_I - U_I* x_in) for U (UPPER) or U'.
+// pk: the pivot tiles' packed triangles, column by column (UPPER) or row by
+// row, so that a step's read is contiguous over the lanes.
+//
+// Bound by latency (a lane walks its row) and, with many block rows, by L1: 16
+// entries in flight need more registers than the compiler grants at the
+// occupancy that the packed triangles allow, hence the bound of 5 CTAs; whole
+// batches go without predicates.  Three FP64 sweeps LEFT / RIGHT: 3000 rows at
+// fill level 1 (24 entries a row, up to some hundred) 71 / 58 us against 114 /
+// 89 with 8 entries and no bound; 300 000 rows of a KKT system 69 / 61 against
+// 92 / 63.
 template <class T, bool UPPER>
-__global__ void __launch_bounds__(32 * kSweepWarps)
+__global__ void __launch_bounds__(32 * kSweepWarps, 5)
     k_sweep_jacobi(int cm, const int* __restrict__ bs, const int2* __restrict__ rng, const int* __restrict__ col,
                    const T* __restrict__ vals, const long long* __restrict__ pk_off,
-                   const int* __restrict__ rowflags, const T* __restrict__ pk_row, const T* __restrict__ b,
+                   const int* __restrict__ rowflags, const T* __restrict__ pk, const T* __restrict__ b,
                    const T* __restrict__ x_in, T* __restrict__ x_out)
 {
     constexpr int kTri = 32 * 33 / 2;
+    constexpr int B = 16;  // a row's entries in flight
     __shared__ T tiles[kSweepWarps][kTri];
     const int warp = threadIdx.x >> 5;
     const int I = blockIdx.x * kSweepWarps + warp;
@@ -607,26 +618,53 @@ __global__ void __launch_bounds__(32 * kSweepWarps)
     if (lane < h) {
         acc = b[fr + lane];
         const int2 kr = rng[fr + lane];
-        for (int k = kr.x; k < kr.y; ++k) acc = fma_rn(-vals[k], x_in[col[k]], acc);
+        int k = kr.x;
+        for (; k + B <= kr.y; k += B) {
+            int c[B];
+            T v[B], xv[B];
+#pragma unroll
+            for (int j = 0; j < B; ++j) {
+                c[j] = col[k + j];
+                v[j] = vals[k + j];
+            }
+#pragma unroll
+            for (int j = 0; j < B; ++j) xv[j] = x_in[c[j]];
+#pragma unroll
+            for (int j = 0; j < B; ++j) acc = fma_rn(-v[j], xv[j], acc);
+        }
+        for (; k < kr.y; k += B) {
+            int c[B];
+            T v[B], xv[B];
+#pragma unroll
+            for (int j = 0; j < B; ++j) {
+                c[j] = (k + j < kr.y) ? col[k + j] : -1;
+                v[j] = (k + j < kr.y) ? vals[k + j] : T(0);
+            }
+#pragma unroll
+            for (int j = 0; j < B; ++j) xv[j] = (c[j] >= 0) ? x_in[c[j]] : T(0);
+#pragma unroll
+            for (int j = 0; j < B; ++j)
+                if (c[j] >= 0) acc = fma_rn(-v[j], xv[j], acc);
+        }
     }
     if (!(rowflags[I] & kRowIdentity)) {
         T* tile = tiles[warp];
-        const T* P = pk_row + pk_off[I];
+        const T* P = pk + pk_off[I];
         for (int e = lane; e < h * (h + 1) / 2; e += 32) tile[e] = P[e];
         __syncwarp();
-        // row r of the triangle at r h - r (r - 1) / 2: columns r .. h - 1
-        auto at = [&](int r, int c) { return tile[r * h - r * (r - 1) / 2 + c - r]; };
-        if (UPPER) {
-            for (int c = h - 1; c >= 0; --c) {
-                if (lane == c) acc = acc / at(c, c);
+        if (UPPER) {  // column by column: column c holds rows 0 .. c
+            const T* column = tile + h * (h - 1) / 2;
+            for (int c = h - 1; c >= 0; column -= c, --c) {
+                if (lane == c) acc = acc / column[c];
                 const T xc = shfl(acc, c);
-                if (lane < c) acc = fma_rn(-at(lane, c), xc, acc);
+                if (lane < c) acc = fma_rn(-column[lane], xc, acc);
             }
-        } else {
-            for (int r = 0; r < h; ++r) {
-                if (lane == r) acc = acc / at(r, r);
+        } else {  // row by row: row r holds columns r .. h - 1
+            const T* row = tile;
+            for (int r = 0; r < h; row += h - 1 - r, ++r) {
+                if (lane == r) acc = acc / row[r];
                 const T xr = shfl(acc, r);
-                if (lane > r && lane < h) acc = fma_rn(-at(r, lane), xr, acc);
+                if (lane > r && lane < h) acc = fma_rn(-row[lane], xr, acc);
             }
         }
     }
@@ -773,7 +811,7 @@ int apply_t(Factor* f, int stage, const void* d_b, void* d_x, cudaStream_t s)
             else
                 k_sweep_jacobi<T, true><<<grid, 32 * kSweepWarps, 0, s>>>(
                     cm, p.d_bs.as<int>(), f->u_rng.as<int2>(), f->u_col.as<int>(), f->u_val.as<T>(),
-                    f->pk_off.as<long long>(), f->rowflags.as<int>(), f->pk_row.as<T>(), rhs, xa, xb);
+                    f->pk_off.as<long long>(), f->rowflags.as<int>(), f->pk_col.as<T>(), rhs, xa, xb);
             std::swap(xa, xb);
         }
         if (left) CULIPX_CUDA(cudaMemcpyAsync(x, xa, n * sizeof(T), cudaMemcpyDeviceToDevice, s));
