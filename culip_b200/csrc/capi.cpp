@@ -338,15 +338,22 @@ CULIPX_API int culipx_factor_info(culipx_factor f, long long* info8)
     long long u_nnz = 0;
     int simple = 0;
     std::vector<int> flags(cm);
-    std::vector<int2> rng(n);
     CULIPX_CUDA(cudaStreamSynchronize(h->stream));
-    CULIPX_CUDA(cudaMemcpy(rng.data(), f->u_rng.get(), n * sizeof(int2), cudaMemcpyDeviceToHost));
-    for (const int2& r : rng) u_nnz += r.y - r.x;
+    if (f->two_level) {  // dropped entries leave gaps, so row by row; all of U' from the first level-1 row on
+        const int g0 = p.bs[p.lvl_rows[p.lvl_off[1]]];
+        std::vector<int2> rng(n - g0);
+        CULIPX_CUDA(cudaMemcpy(rng.data(), f->ut_rng.as<int2>() + g0, rng.size() * sizeof(int2), cudaMemcpyDeviceToHost));
+        for (const int2& r : rng) u_nnz += r.y - r.x;
+    } else {
+        int end = 0;
+        CULIPX_CUDA(cudaMemcpy(&end, f->u_off.as<int>() + n, sizeof(int), cudaMemcpyDeviceToHost));
+        u_nnz = end;
+    }
     CULIPX_CUDA(cudaMemcpy(&simple, f->scan_s.as<int>() + cm, sizeof(int), cudaMemcpyDeviceToHost));
     if (cm) CULIPX_CUDA(cudaMemcpy(flags.data(), f->rowflags.get(), cm * sizeof(int), cudaMemcpyDeviceToHost));
-    std::vector<int> extra(p.coarse_nnz, 0);
-    if (p.coarse_nnz && !f->two_level)
-        CULIPX_CUDA(cudaMemcpy(extra.data(), f->got_extra.get(), p.coarse_nnz * sizeof(int), cudaMemcpyDeviceToHost));
+    std::vector<int> extra(f->two_level ? 0 : p.coarse_nnz);
+    if (!extra.empty())
+        CULIPX_CUDA(cudaMemcpy(extra.data(), f->got_extra.get(), extra.size() * sizeof(int), cudaMemcpyDeviceToHost));
     long long granted = 0;
     for (int v : extra) granted += (v > 0);
     long long tiles = 0, tile_slots = 0, two = 0;
