@@ -6,6 +6,7 @@
 #include <atomic>
 #include <cmath>
 #include <cstdlib>
+#include <memory>
 
 namespace culipx {
 
@@ -450,7 +451,7 @@ int batch_create(culipx_handle_t* h, const Pattern* p, int num, const int* h_row
             else if (e0 != q) return fail(CULIPX_INVALID_ARG, "culipx_batch_create: level list not grouped by system");
             e0 = q + 1;
         }
-    auto* bt = new culipx_batch_t();
+    auto bt = std::make_unique<culipx_batch_t>();
     bt->h = h;
     bt->pat = p;
     bt->num = num;
@@ -462,11 +463,8 @@ int batch_create(culipx_handle_t* h, const Pattern* p, int num, const int* h_row
     if (st == CULIPX_OK) st = bt->d_out.alloc(h, (size_t)num * 8 * sizeof(double));
     if (st == CULIPX_OK) st = bt->d_next.alloc(h, sizeof(int));
     if (st == CULIPX_OK && p->two_level) st = lockstep_plan(h, *p, num, h_row_off, qb, qe, bt->lock);
-    if (st != CULIPX_OK) {
-        delete bt;
-        return st;
-    }
-    *out = bt;
+    if (st != CULIPX_OK) return st;
+    *out = bt.release();
     return CULIPX_OK;
 }
 

@@ -18,6 +18,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <memory>
 #include <new>
 #include <numeric>
 
@@ -296,7 +297,7 @@ int analyze_pattern(culipx_handle_t* h, int n, const int* rowptr, const int* col
         return fail(CULIPX_INVALID_ARG, "culipx_pattern_analyze: bad precision");
     if (rowptr[0] != 0) return fail(CULIPX_INVALID_ARG, "culipx_pattern_analyze: rowptr[0] != 0");
 
-    auto* pp = new culipx_pattern_t();
+    auto pp = std::make_unique<culipx_pattern_t>();  // freed on every way out, exceptions too
     Pattern& p = *pp;
     p.handle = h;
     p.n = n;
@@ -311,28 +312,22 @@ int analyze_pattern(culipx_handle_t* h, int n, const int* rowptr, const int* col
     p.bs.push_back(n);
     for (int b = 0; b < cm; ++b) {
         const int sz = p.bs[b + 1] - p.bs[b];
-        if (sz < 1 || sz > 32) {
-            delete pp;
+        if (sz < 1 || sz > 32)
             return fail(CULIPX_INVALID_ARG, "culipx_pattern_analyze: block %d has size %d (must be 1..32)", b, sz);
-        }
     }
-    if (p.bs[0] != 0) { delete pp; return fail(CULIPX_INVALID_ARG, "culipx_pattern_analyze: block_starts[0] != 0"); }
+    if (p.bs[0] != 0) return fail(CULIPX_INVALID_ARG, "culipx_pattern_analyze: block_starts[0] != 0");
     // systems of a block-diagonal union (default: one system): per block row
     // its system's first block row and block count, for the format rule
     std::vector<int> sys_first(cm, 0), sys_blocks(cm, cm);
     if (num_systems > 1 && system_row_offsets) {
-        if (system_row_offsets[0] != 0 || system_row_offsets[num_systems] != n) {
-            delete pp;
+        if (system_row_offsets[0] != 0 || system_row_offsets[num_systems] != n)
             return fail(CULIPX_INVALID_ARG, "culipx_pattern_analyze_systems: row offsets must run from 0 to n");
-        }
         int b0 = 0;
         for (int k = 0; k < num_systems; ++k) {
             int b1 = b0;
             while (b1 < cm && p.bs[b1] < system_row_offsets[k + 1]) ++b1;
-            if (p.bs[b0] != system_row_offsets[k] || p.bs[b1] != system_row_offsets[k + 1] || b1 == b0) {
-                delete pp;
+            if (p.bs[b0] != system_row_offsets[k] || p.bs[b1] != system_row_offsets[k + 1] || b1 == b0)
                 return fail(CULIPX_INVALID_ARG, "culipx_pattern_analyze_systems: system %d does not start and end on block boundaries", k);
-            }
             for (int I = b0; I < b1; ++I) {
                 sys_first[I] = b0;
                 sys_blocks[I] = b1 - b0;
@@ -343,10 +338,8 @@ int analyze_pattern(culipx_handle_t* h, int n, const int* rowptr, const int* col
     for (int i = 0; i < n; ++i) p.longest_row = std::max(p.longest_row, rowptr[i + 1] - rowptr[i]);
     for (int i = 0; i < n; ++i)
         for (int q = rowptr[i]; q < rowptr[i + 1]; ++q)
-            if (colidx[q] < 0 || colidx[q] >= n || (q > rowptr[i] && colidx[q] <= colidx[q - 1])) {
-                delete pp;
+            if (colidx[q] < 0 || colidx[q] >= n || (q > rowptr[i] && colidx[q] <= colidx[q - 1]))
                 return fail(CULIPX_INVALID_ARG, "culipx_pattern_analyze: row %d: columns must be sorted, unique, in range", i);
-            }
     p.row_block.resize(n);
     for (int b = 0; b < cm; ++b)
         for (int j = p.bs[b]; j < p.bs[b + 1]; ++j) p.row_block[j] = b;
@@ -490,7 +483,7 @@ int analyze_pattern(culipx_handle_t* h, int n, const int* rowptr, const int* col
             d.val_off = (int)o;
             o += d.cap;
             if (p.fmt[q] == kSparse) p.sparse_slots += d.cap;
-            if (o > 0x7fffffffLL) { delete pp; return fail(CULIPX_NOT_SUPPORTED, "culipx_pattern_analyze: factor storage exceeds 2^31 slots"); }
+            if (o > 0x7fffffffLL) return fail(CULIPX_NOT_SUPPORTED, "culipx_pattern_analyze: factor storage exceeds 2^31 slots");
         }
         p.val_slots = o;
     }
@@ -505,7 +498,7 @@ int analyze_pattern(culipx_handle_t* h, int n, const int* rowptr, const int* col
 
     // device mirror (not for a host-only handle)
     if (h->device < 0) {
-        *out = pp;
+        *out = pp.release();
         return CULIPX_OK;
     }
     int st = CULIPX_OK;
@@ -555,9 +548,9 @@ int analyze_pattern(culipx_handle_t* h, int n, const int* rowptr, const int* col
         p.two_tiles = reinterpret_cast<const two::Tile*>(d + at[8]);
         p.two_pairs = reinterpret_cast<const uint2*>(d + at[9]);
     }
-    if (st != CULIPX_OK) { delete pp; return st; }
+    if (st != CULIPX_OK) return st;
     p.device_bytes += (long long)p.d_two.bytes();
-    *out = pp;
+    *out = pp.release();
     return CULIPX_OK;
 }
 
