@@ -1006,6 +1006,8 @@ int factor_create(Pattern* p, Factor** out)
         al(f->kind, (cm + 15) / 16 * 16);
         al(f->u_sub, (size_t)n * f->vbytes);
         al(f->u_pair, 2 * (size_t)p->two_entries * f->vbytes);
+        const int zero = 0;
+        if (st == CULIPX_OK) st = f->nonfinite.upload(h, &zero, sizeof(int));
     }
     al(f->work, (size_t)n * f->vbytes);
     if (st == CULIPX_OK) st = f->pk_off.upload(h, p->pk_off.data(), (cm + 1) * sizeof(long long));
@@ -1182,7 +1184,8 @@ int export_two_level(Factor* f, int* blk_nnz, long long* blk_off, int* idx, void
         CULIPX_CUDA(cudaMemcpyAsync(col.data(), f->u_col.get(), slots * sizeof(int), cudaMemcpyDeviceToHost, s));
         CULIPX_CUDA(cudaMemcpyAsync(uv.data(), f->u_val.get(), slots * vb, cudaMemcpyDeviceToHost, s));
     }
-    std::vector<unsigned char> sub(n * vb);
+    std::vector<unsigned char> sub(n * vb), pivots(3 * (size_t)n * vb);
+    CULIPX_CUDA(cudaMemcpyAsync(pivots.data(), f->tri.get(), pivots.size(), cudaMemcpyDeviceToHost, s));
     CULIPX_CUDA(cudaMemcpyAsync(sub.data(), f->u_sub.get(), sub.size(), cudaMemcpyDeviceToHost, s));
     CULIPX_CUDA(cudaMemcpyAsync(pk.data(), f->pk_row.get(), pk.size(), cudaMemcpyDeviceToHost, s));
     CULIPX_CUDA(cudaStreamSynchronize(s));
@@ -1193,6 +1196,23 @@ int export_two_level(Factor* f, int* blk_nnz, long long* blk_off, int* idx, void
     auto put = [&](long long at, const unsigned char* v) {
         if (val) std::memcpy((unsigned char*)val + at * vb, v, vb);
     };
+    // a tile's entries left of a 1x1 pivot are 0 / pivot, those of a 2x2 pivot 0
+    auto left_of = [&](size_t g) {
+        double d[3];
+        for (int k = 0; k < 3; ++k) {
+            if (vb == 8) std::memcpy(&d[k], &pivots[(3 * g + k) * 8], 8);
+            else {
+                float v;
+                std::memcpy(&v, &pivots[(3 * g + k) * 4], 4);
+                d[k] = v;
+            }
+        }
+        return std::isnan(d[1]) && d[0] == 0.0 && d[2] == 0.0;
+    };
+    const double nan64 = std::nan("");
+    const float nan32 = std::nanf("");
+    const unsigned char* const nan_bytes =
+        vb == 8 ? (const unsigned char*)&nan64 : (const unsigned char*)&nan32;
     long long o = 0;
     std::vector<int> next(32);
     for (int b = 0; b < cnz; ++b) {
@@ -1213,6 +1233,8 @@ int export_two_level(Factor* f, int* blk_nnz, long long* blk_off, int* idx, void
         if (I == J) {
             for (int i = 0; i < r; ++i) {
                 if (i > 0 && (flags[I] & kRowHas2x2)) put(o + i * r + i - 1, &sub[(size_t)(fr + i) * vb]);
+                if (!(flags[I] & kRowIdentity) && left_of(fr + i))
+                    for (int j = 0; j < i; ++j) put(o + i * r + j, nan_bytes);
                 for (int j = i; j < r; ++j) {
                     if (!(flags[I] & kRowIdentity))
                         put(o + i * r + j, &pk[(pko[I] + i * r - i * (i - 1) / 2 + j - i) * vb]);

@@ -63,6 +63,7 @@ struct Factor {
     // factor_two_level.cu: a byte per level-1 block row; u and D u per entry;
     // in block rows with 2x2 pivots the pivot tile's subdiagonal (export only)
     DeviceBuffer kind, u_pair, u_sub;
+    DeviceBuffer nonfinite;              // 1 while a factorization has met a level-0 pivot that is not finite
     DeviceBuffer u_rng, ut_rng;          // per fine row its entries' [first, end), as int2
     DeviceBuffer piv_off;                // per block row: value slot of its pivot tile
     // the persistent solver's copies: upper triangles of the non-identity

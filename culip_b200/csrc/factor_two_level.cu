@@ -18,7 +18,8 @@
 // Every value and every order of summation is the general path's: an update
 // block's contributions to a tile entry are summed in row order and then
 // subtracted, blocks in row order; entries of sparse blocks with |u| <= NZ_EPS
-// are dropped.
+// are dropped.  Zeros that the general path multiplies with a NaN or an
+// infinity are not in K's rows: spread_nonfinite puts their NaN in.
 //
 // Bound: the tiles' serial pivot steps (short scoreboard and fixed latency, an
 // issue slot in three used), not bandwidth.  Measured on the scale system
@@ -96,6 +97,8 @@ struct TwoArgs {
     int* cplx;
     CItem* citem;
     unsigned char* kind;  // per level-1 block row: its rows if simple, else 0
+    int* nonfinite;       // set by the rows, cleared by the last kernel
+    int blocks;
 };
 
 // a level-0 pivot from K's diagonal entry (0 if K stores none), perturbed as
@@ -127,6 +130,7 @@ __global__ void __launch_bounds__(256) k_two_rows(TwoArgs<T> a)
     after_previous();  // K's values; what stands above is the pattern's
     if (i >= a.n0) return;
     const T d11 = level0_pivot(a, tagged, k0);
+    if (!isfinite(d11)) *a.nonfinite = 1;
     const T d22 = (tagged & two::kNextInBlock) ? level0_pivot(a, __ldg(a.l0_rows + i + 1), k1) : T(0);
     const T d12 = T(0);
     const T gr = sqrt(fma_rn(d11, d11, d12 * d12));
@@ -161,6 +165,47 @@ __global__ void __launch_bounds__(256) k_two_rows(TwoArgs<T> a)
     a.perm[g] = g;
     a.is_piv[g] = 1;
     a.simple_rows[i] = g;
+}
+
+// What the general path's update of a tile by a whole block gives beyond the
+// entries of K's rows where values are not finite (0 x inf and 0 x NaN are
+// NaN): with lv = D u its factor for row a of the tile,
+//   * a pivot of the block that is not finite makes lv NaN in every row a that
+//     has an entry in the block, and a NaN or, next to other rows of the block,
+//     an infinite entry does so in its own row: the tile's row is NaN;
+//   * an infinite lv otherwise meets the zeros of U's row: the places of the
+//     tile's row that are still finite are NaN.
+// A lane looks through its row's entries; reached only with such values.
+template <class T>
+__device__ void spread_nonfinite(const TwoArgs<T>& a, T* tile, int h, int k0, int k1)
+{
+    const int b = lane_id();
+    bool all = false, rest = false;
+#pragma unroll 1
+    for (int k = k0; k < k1; ++k) {
+        const int2 w = __ldg(a.low + k);
+        const auto q = a.up[w.y];
+        if (q.x == T(0)) continue;  // dropped
+        const int g = w.x & two::kColMask;
+        int lo = 0, hi = a.blocks;  // the block row that holds g
+        while (hi - lo > 1) {
+            const int mid = (lo + hi) / 2;
+            if (__ldg(a.bs + mid) <= g) lo = mid;
+            else hi = mid;
+        }
+        const int g0 = __ldg(a.bs + lo), g1 = __ldg(a.bs + lo + 1);
+        bool pivots = true;
+#pragma unroll 1
+        for (int r = g0; r < g1; ++r) pivots &= (bool)isfinite(a.dg[r]);
+        all |= !pivots || q.x != q.x || q.y != q.y || (g1 - g0 > 1 && !isfinite(q.x));
+        rest |= !isfinite(q.x) || !isfinite(q.y);
+    }
+    const unsigned alls = __ballot_sync(0xffffffffu, all), rests = __ballot_sync(0xffffffffu, rest);
+    const T nan = T(0) / T(0);
+    for (int r = 0; r < h; ++r) {
+        T* const at = tile + r * kTileStride + b;
+        if (b < h && (((alls >> r) & 1u) || (((rests >> r) & 1u) && isfinite(*at)))) *at = nan;
+    }
 }
 
 // One level-1 block row per warp, the upper triangle T_ab at tile[a][b].  Lane b
@@ -264,6 +309,7 @@ __global__ void __launch_bounds__(32 * kTileWarps, 6) k_two_tiles(TwoArgs<T> a)
     }
     __syncwarp();
     if (b < h) tile[b * kTileStride + b] = diag - sum;
+    const bool spoilt = __any_sync(0xffffffffu, *a.nonfinite || (b < h && !isfinite(diag - sum)));
     const int p0 = d1.y, p1 = __ldg(&a.tiles[t + 1].pair);
     for (int i = p0 + b; i < p1; i += 32) {
         uint2 m = __ldg(a.pairs + i);
@@ -286,6 +332,10 @@ __global__ void __launch_bounds__(32 * kTileWarps, 6) k_two_tiles(TwoArgs<T> a)
             add();
         }
         *at = v - s;
+    }
+    if (spoilt) {
+        __syncwarp();
+        spread_nonfinite(a, tile, h, k0, k1);
     }
     // the sweeps read a tile's run of slots whole
     for (int q = ut; q < k1; ++q) {
@@ -445,6 +495,7 @@ template <class T>
 __global__ void __launch_bounds__(kOrderT) k_two_order(TwoArgs<T> a, int splits)
 {
     after_previous();
+    if (blockIdx.x == 0 && threadIdx.x == 0) *a.nonfinite = 0;  // the tiles have read it
     if ((int)blockIdx.x < splits) {
         split_rows(a, blockIdx.x * kOrderT);
         return;
@@ -556,6 +607,8 @@ int run(Factor* f, const void* d_vals, cudaStream_t s, int* launches)
     a.cplx = f->cplx.as<int>();
     a.citem = f->citem.as<CItem>();
     a.kind = f->kind.as<unsigned char>();
+    a.nonfinite = f->nonfinite.as<int>();
+    a.blocks = p.num_blocks;
     CULIPX_TRY(launch_overlapped(k_two_rows<T>, dim3((a.n0 + 255) / 256), dim3(256), s, !f->capturing, a));
     CULIPX_TRY(launch_overlapped(k_two_tiles<T>, dim3((a.nr1 + kTileWarps - 1) / kTileWarps), dim3(32 * kTileWarps),
                                  s, !f->capturing, a));

@@ -22,7 +22,8 @@ WRITTEN = {
                 "k_long_rows": ["x", "y"]},
     "kkt_assembly.cu": {"k_kkt_values": ["aval", "x", "s", "d", "kval"]},
     "solve.cu": {"k_solve_D": ["in", "out"]},
-    "factor_two_level.cu": {"level0_pivot": ["kval"], "k_two_rows": ["kval"], "k_two_tiles": ["up"],
+    "factor_two_level.cu": {"level0_pivot": ["kval"], "k_two_rows": ["kval"], "spread_nonfinite": ["up", "dg"],
+                            "k_two_tiles": ["up", "nonfinite"],
                             "split_rows": ["kind", "kinds", "rowflags", "ndmask"], "k_two_order": ["up", "iperm"]},
     "apply_two_level.cu": {"k_two_left": ["b", "x"], "k_two_right_tiles": ["b", "x"], "k_two_right_rows": ["b", "x"]},
 }
