@@ -19,6 +19,12 @@
 // on the others, on its place in the batch or on the grid: its sums are taken
 // by one CTA over the rows' stored terms.
 //
+// The iterations end when no system of more than kLockRows rows is left: the
+// small ones, whose count may be many times the large ones', go on in
+// k_sqmr_rest with a CTA each (one easy system of 30 000 rows and 40 hard ones
+// of 450: 17.0 ms all on the grid, 9.2 so, 22.5 with a CTA each from the start;
+// of 9000 rows and 100 of 450: 23.7, 9.0 and 7.7).
+//
 // Bound: HBM for the factor, K and the vectors of all systems (their working
 // set is beyond L2), then the dependent loads of a tile's chain.
 #include "sqmr_persistent.cuh"
@@ -29,14 +35,6 @@ namespace culipx {
 namespace persistent {
 
 namespace {
-
-// one system's coefficients, read by the units of the next phase
-struct alignas(16) LockCoef {
-    double na, nb;              // U sweep: -alpha, -beta_k
-    double sc;                  // 1 / delta (the scale of level-0 Av)
-    double nbrr, ne, ir, tau;   // p / x update
-    int act, pad;               // still iterating
-};
 
 struct LockArgs {
     int num, chunks, tiles;
@@ -49,9 +47,14 @@ struct LockArgs {
     double* dv;
     Scal* scal;
     LockCoef* coef;
-    int* active;        // systems still iterating
+    int* active;        // [0] systems of more than kLockRows rows still iterating, [1] iterations taken
     double* out;        // num x 8
 };
+
+__device__ __forceinline__ bool large(const LockArgs& k, int s)
+{
+    return __ldg(k.row_off + s + 1) - __ldg(k.row_off + s) > kLockRows;
+}
 
 template <class TF>
 __device__ __forceinline__ ItemMeta meta_of_tile(const PArgs<TF>& a, const int4& t)
@@ -255,7 +258,7 @@ __global__ void __launch_bounds__(kT, kCtasPerSm) k_sqmr_lockstep(PArgs<TF> a, L
             C.nb = -Q.beta[0];
             C.sc = 1.0;  // the scale of the Av that the initial phase leaves
             C.act = !Q.done;
-            if (!Q.done) atomicAdd(k.active, 1);
+            if (!Q.done && large(k, s)) atomicAdd(k.active, 1);
         }
         __syncthreads();
     }
@@ -399,7 +402,7 @@ __global__ void __launch_bounds__(kT, kCtasPerSm) k_sqmr_lockstep(PArgs<TF> a, L
                 C.nb = -Q.beta[k1];
                 if (Q.done) {
                     C.act = 0;
-                    atomicSub(k.active, 1);
+                    if (large(k, s)) atomicSub(k.active, 1);
                 }
             }
             __syncthreads();
@@ -408,7 +411,8 @@ __global__ void __launch_bounds__(kT, kCtasPerSm) k_sqmr_lockstep(PArgs<TF> a, L
         ++it;
     }
 
-    // ---- x = P U^-1 D^-1 x~ ----
+    if (blockIdx.x == 0 && tid == 0) k.active[1] = it;
+    // ---- x = P U^-1 D^-1 x~ (k_sqmr_rest writes that of an unfinished system again) ----
     for (int t = wid; t < k.tiles; t += nw) {
         const ItemMeta m = meta_of_tile(a, __ldg(k.tile + t));
         const double y[1] = {(lane < m.h) ? a.xt[m.fr + lane] : 0.0};
@@ -445,27 +449,33 @@ size_t lockstep_bytes(int n, int num)
 }
 
 template <class TF>
-int lockstep_launch(const PArgs<TF>& a, const LockPlan& p, int num, const int* row_off, const int* qb, const int* qe,
-                    void* work, double* out, int grid, cudaStream_t s)
+int lockstep_launch(const PArgs<TF>& a, const LockPlan& p, const BatchArgs& bt, void* work, int grid, int rest_grid,
+                    cudaStream_t s)
 {
     LockArgs k;
-    k.num = num;
+    k.num = bt.num;
     k.chunks = p.chunks;
     k.tiles = p.tiles;
     k.chunk = p.units.as<int4>();
     k.tile = k.chunk + p.chunks;
-    k.row_off = row_off;
-    k.qb = qb;
-    k.qe = qe;
+    k.row_off = bt.row_off;
+    k.qb = bt.qb;
+    k.qe = bt.qe;
     k.coef = static_cast<LockCoef*>(work);
-    k.scal = reinterpret_cast<Scal*>(k.coef + num);
-    k.da = reinterpret_cast<double*>(k.scal + num);
+    k.scal = reinterpret_cast<Scal*>(k.coef + bt.num);
+    k.da = reinterpret_cast<double*>(k.scal + bt.num);
     k.dv = k.da + a.n;
     k.active = reinterpret_cast<int*>(k.dv + a.n);
-    k.out = out;
+    k.out = bt.out;
     CULIPX_CUDA(cudaMemsetAsync(k.active, 0, sizeof(int), s));
+    CULIPX_CUDA(cudaMemsetAsync(bt.next, 0, sizeof(int), s));
     void* args[] = {const_cast<PArgs<TF>*>(&a), &k};
     CULIPX_CUDA(cudaLaunchCooperativeKernel((const void*)k_sqmr_lockstep<TF>, dim3(grid), dim3(kT), args, 0, s));
+    const Scal* scal = k.scal;
+    const LockCoef* coef = k.coef;
+    const int* at = k.active + 1;
+    void* rest[] = {const_cast<PArgs<TF>*>(&a), const_cast<BatchArgs*>(&bt), &scal, &coef, &at};
+    CULIPX_CUDA(cudaLaunchKernel(rest_fn<TF>(), dim3(rest_grid), dim3(kT), rest, 0, s));
     return CULIPX_OK;
 }
 
@@ -475,10 +485,10 @@ const void* lockstep_kernel()
     return (const void*)k_sqmr_lockstep<TF>;
 }
 
-template int lockstep_launch<double>(const PArgs<double>&, const LockPlan&, int, const int*, const int*, const int*, void*,
-                                     double*, int, cudaStream_t);
-template int lockstep_launch<float>(const PArgs<float>&, const LockPlan&, int, const int*, const int*, const int*, void*,
-                                     double*, int, cudaStream_t);
+template int lockstep_launch<double>(const PArgs<double>&, const LockPlan&, const BatchArgs&, void*, int, int,
+                                     cudaStream_t);
+template int lockstep_launch<float>(const PArgs<float>&, const LockPlan&, const BatchArgs&, void*, int, int,
+                                    cudaStream_t);
 template const void* lockstep_kernel<double>();
 template const void* lockstep_kernel<float>();
 

@@ -317,7 +317,7 @@ namespace {
 
 // The whole-grid solve (a two-level factor, A on its pattern).
 template <class TF>
-int launch_lockstep(Batch* bt, const PArgs<TF>& a, Sqmr* w)
+int launch_lockstep(Batch* bt, const PArgs<TF>& a, const BatchArgs& ba, int rest_grid, Sqmr* w)
 {
     culipx_handle_t* h = bt->h;
     const size_t need = lockstep_bytes(a.n, bt->num);
@@ -335,9 +335,8 @@ int launch_lockstep(Batch* bt, const PArgs<TF>& a, Sqmr* w)
             return (int)CULIPX_OK;
         },
         &G));
-    CULIPX_TRY(lockstep_launch<TF>(a, bt->lock, bt->num, bt->d_row_off.as<int>(), bt->d_qb.as<int>(),
-                                   bt->d_qe.as<int>(), w->lock.get(), bt->d_out.as<double>(), G, h->stream));
-    h->launches += 1;
+    CULIPX_TRY(lockstep_launch<TF>(a, bt->lock, ba, w->lock.get(), G, rest_grid, h->stream));
+    h->launches += 2;
     return CULIPX_OK;
 }
 
@@ -371,7 +370,7 @@ int launch_batched(Batch* bt, Csr* A, Factor* M, const double* b, double* x, dou
     ba.next = bt->d_next.as<int>();
     CULIPX_TRY(zero_vectors(a, 1, s));
     // static pivots or a threshold leave a factor whose level 0 is not known to be simple
-    if (bt->lock.use && M->two_level && a.fuse_l0) return launch_lockstep<TF>(bt, a, w);
+    if (bt->lock.use && M->two_level && a.fuse_l0) return launch_lockstep<TF>(bt, a, ba, std::min(G, bt->num), w);
     CULIPX_CUDA(cudaMemsetAsync(ba.next, 0, sizeof(int), s));
     void* args[] = {&a, &ba};
     CULIPX_CUDA(cudaLaunchKernel(batched_fn<TF>(), dim3(std::min(G, bt->num)), dim3(kT), args, 0, s));
@@ -389,14 +388,15 @@ namespace {
 // 60 for its synchronisations, 0.15 per 1000 rows of all systems and 2.4 per
 // 1000 rows of the largest for its sums.  256 systems of 750 to 30 000 rows:
 // 0.84 ms against 0.46; one system of 30 000 rows: 0.55 against 0.09; 296
-// systems of 4500 rows: 0.20 against 0.29, which keep a CTA each.  Both kernels
-// give the same bits, so the choice does not show in the results.
+// systems of 4500 rows: 0.20 against 0.29, which keep a CTA each.  Small systems
+// that outlast the large ones get a CTA each from there on (k_sqmr_rest).  Both
+// kernels give the same bits, so the choice does not show in the results.
 int lockstep_plan(culipx_handle_t* h, const Pattern& p, int num, const int* row_off, const std::vector<int>& qb,
                   const std::vector<int>& qe, LockPlan& plan)
 {
     int largest = 0;
     for (int s = 0; s < num; ++s) largest = std::max(largest, row_off[s + 1] - row_off[s]);
-    plan.use = 25.0 + 17.5e-3 * largest > 60.0 + 0.15e-3 * p.n + 2.4e-3 * largest;
+    plan.use = largest > kLockRows && 25.0 + 17.5e-3 * largest > 60.0 + 0.15e-3 * p.n + 2.4e-3 * largest;
     if (!plan.use) return CULIPX_OK;
     std::vector<int4> chunk, tile;
     int pos = 0;  // level 0's fine rows in level-list order

@@ -1011,9 +1011,11 @@ __device__ __forceinline__ LvlBounds level_bounds(const PArgs<TF>& a, const SysV
     return LvlBounds{__ldg(a.scan_c + q0), __ldg(a.scan_c + q1), __ldg(a.scan_s + q0), __ldg(a.scan_s + q1)};
 }
 
-template <class TF, int NR, class Ctx>
+// REST: a solve that another kernel began (k_sqmr_lockstep), from iteration it0
+// on: S and the vectors hold its state, sc0 the scale of its level-0 Av.
+template <class TF, int NR, class Ctx, bool REST = false>
 __device__ void sqmr_body(const PArgs<TF>& a, Ctx& ctx, const SysView& sv, Scal (&S)[NR], double (*sh)[kW],
-                          ResSlot<TF>* slots = nullptr)
+                          ResSlot<TF>* slots = nullptr, int it0 = 0, double sc0 = 1.0)
 {
     const int tid = threadIdx.x, lane = (int)lane_id();
     const int wid = ctx.wid, nwarps = ctx.nwarps;
@@ -1024,9 +1026,11 @@ __device__ void sqmr_body(const PArgs<TF>& a, Ctx& ctx, const SysView& sv, Scal 
     if (tid < kLvlCache && tid < a.nl) lvb[tid] = level_bounds(a, sv, tid);
     if (tid == 0) {
         for (int j = 0; j < NR; ++j) {
-            memset(&S[j], 0, sizeof(Scal));
-            S[j].c[0] = -1.0;
-            cfs.sc[j] = 1.0;  // the scale of the Av that the initial phase leaves
+            if constexpr (!REST) {
+                memset(&S[j], 0, sizeof(Scal));
+                S[j].c[0] = -1.0;
+            }
+            cfs.sc[j] = REST ? sc0 : 1.0;  // the scale of the Av that the initial phase leaves
         }
         long long np = 0;
         for (int L = 1; L < a.nl; ++L) {
@@ -1118,7 +1122,7 @@ __device__ void sqmr_body(const PArgs<TF>& a, Ctx& ctx, const SysView& sv, Scal 
     __syncthreads();
 
     // ---- init: v0 = U'^-1 P' b; ||v0|| ----
-    {
+    if constexpr (!REST) {
         double one[NR];
 #pragma unroll
         for (int j = 0; j < NR; ++j) one[j] = 1.0;
@@ -1132,7 +1136,7 @@ __device__ void sqmr_body(const PArgs<TF>& a, Ctx& ctx, const SysView& sv, Scal 
             ctx.sync();
         }
     }
-    {
+    if constexpr (!REST) {
         double r[NR];
 #pragma unroll
         for (int j = 0; j < NR; ++j) r[j] = 0.0;
@@ -1152,7 +1156,7 @@ __device__ void sqmr_body(const PArgs<TF>& a, Ctx& ctx, const SysView& sv, Scal 
     double ww[NR];
 #pragma unroll
     for (int j = 0; j < NR; ++j) ww[j] = 0.0;
-    {
+    if constexpr (!REST) {
         double inv_pb[NR];
 #pragma unroll
         for (int j = 0; j < NR; ++j) inv_pb[j] = S[j].inv_pb;
@@ -1179,7 +1183,7 @@ __device__ void sqmr_body(const PArgs<TF>& a, Ctx& ctx, const SysView& sv, Scal 
         }
     }
     // Av = U'^-1 P' K ev; alpha's dots for iteration 0; eta_0 = 1/||D^-1 v0||
-    {
+    if constexpr (!REST) {
         double r[3 * NR];
         double one[NR];
 #pragma unroll
@@ -1226,7 +1230,7 @@ __device__ void sqmr_body(const PArgs<TF>& a, Ctx& ctx, const SysView& sv, Scal 
 
     // the counted iteration has no ctx.sync() between here and the loop's end
     if (counted && a.count_red) ctx.begin_counted(a.lvl_done, a.red_skew);
-    int it = 0;
+    int it = REST ? it0 : 0;
     for (;;) {
         bool any = false;
 #pragma unroll
@@ -1604,6 +1608,41 @@ __global__ void __launch_bounds__(kT, kCtasPerSm) k_sqmr_batched(PArgs<TF> a, Ba
     }
 }
 
+// One system's coefficients in k_sqmr_lockstep, read by the units of the next
+// phase
+struct alignas(16) LockCoef {
+    double na, nb;              // U sweep: -alpha, -beta_k
+    double sc;                  // 1 / delta (the scale of level-0 Av)
+    double nbrr, ne, ir, tau;   // p / x update
+    int act, pad;               // still iterating
+};
+
+// The systems that k_sqmr_lockstep left unfinished (small ones, once every
+// larger system has stopped), a CTA each from its iteration `at` on.
+template <class TF>
+__global__ void __launch_bounds__(kT, kCtasPerSm)
+    k_sqmr_rest(PArgs<TF> a, BatchArgs bt, const Scal* scal, const LockCoef* coef, const int* at)
+{
+    __shared__ Scal S[1];
+    __shared__ double sh[kMaxNV][kW];
+    __shared__ int sys;
+    CtaCtx ctx{(int)(threadIdx.x >> 5), kW, (int)threadIdx.x, kT};
+    const int it0 = *at;
+    if (it0 >= a.max_it) return;
+    for (;;) {
+        if (threadIdx.x == 0) sys = atomicAdd(bt.next, 1);
+        __syncthreads();
+        const int s = sys;
+        __syncthreads();
+        if (s >= bt.num) break;
+        if (!coef[s].act) continue;
+        if (threadIdx.x == 0) S[0] = scal[s];
+        const SysView sv{__ldg(bt.row_off + s), __ldg(bt.row_off + s + 1), bt.qb + (size_t)s * a.nl,
+                         bt.qe + (size_t)s * a.nl, bt.out + (size_t)s * 8};
+        sqmr_body<TF, 1, CtaCtx, true>(a, ctx, sv, S, sh, nullptr, it0, coef[s].sc);
+    }
+}
+
 // Batched solves of independent systems that each have their own pattern,
 // factor, matrix and vectors (the serving path): the CTA copies system s's
 // argument block into shared memory and runs the same body over its rows,
@@ -1648,6 +1687,8 @@ template <class TF, int CTAS, int NR>
 const void* persistent_fn();
 template <class TF>
 const void* batched_fn();
+template <class TF>
+const void* rest_fn();
 template <class TF, bool MULTI>
 const void* many_fn();
 
@@ -1659,6 +1700,7 @@ const void* many_fn();
     template <> const void* persistent_fn<TF, 1, 4>();     \
     template <> const void* persistent_fn<TF, 2, 4>();     \
     template <> const void* batched_fn<TF>();              \
+    template <> const void* rest_fn<TF>();                 \
     template <> const void* many_fn<TF, false>();          \
     template <> const void* many_fn<TF, true>();
 CULIPX_SQMR_DECLARE(double)
@@ -1675,6 +1717,12 @@ CULIPX_SQMR_DECLARE(float)
     const void* batched_fn<TF>()               \
     {                                          \
         return (const void*)k_sqmr_batched<TF>; \
+    }
+#define CULIPX_SQMR_REST(TF)                \
+    template <>                             \
+    const void* rest_fn<TF>()               \
+    {                                       \
+        return (const void*)k_sqmr_rest<TF>; \
     }
 #define CULIPX_SQMR_MANY(TF, MULTI)                \
     template <>                                    \
