@@ -222,10 +222,9 @@ __global__ void __launch_bounds__(32 * kApplyWarps) k_two_right_tiles(ApplyArgs<
     if (lane < h) a.x[to] = acc;
 }
 
-template <class T>
+template <class T, int B>
 __global__ void __launch_bounds__(256) k_two_right_rows(ApplyArgs<T> a)
 {
-    constexpr int B = 8;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const bool in = i < a.n0;
     int g = 0;
@@ -286,7 +285,13 @@ int apply(Factor* f, bool left, const void* d_b, void* d_x, cudaStream_t s)
         return launch_overlapped(k_two_left<T>, dim3(tile_ctas + copies), dim3(32 * kApplyWarps), s, true, a, tile_ctas);
     }
     CULIPX_TRY(launch_overlapped(k_two_right_tiles<T>, dim3(tile_ctas), dim3(32 * kApplyWarps), s, true, a));
-    return launch_overlapped(k_two_right_rows<T>, dim3((a.n0 + 255) / 256), dim3(256), s, true, a);
+    // a thread per row: fewer rows than fill the device are spread over it, as
+    // a long row is its thread's serial chain (3000 rows of 200 entries, FP64:
+    // 45 us for RIGHT with CTAs of 256, 27 with the general sweeps)
+    const int threads = std::min(256, std::max(32, (a.n0 / (4 * 148) + 31) / 32 * 32));
+    const dim3 grid((a.n0 + threads - 1) / threads), block(threads);
+    if (p.two_entries > 12LL * a.n0) return launch_overlapped(k_two_right_rows<T, 16>, grid, block, s, true, a);
+    return launch_overlapped(k_two_right_rows<T, 8>, grid, block, s, true, a);
 }
 
 }  // namespace
