@@ -1,7 +1,7 @@
 """Kernels that are launched over their predecessor's end (csrc/launch.cuh).
 
 Their life begins before the predecessor has finished writing.  Each has to
-wait (after_previous), and what the predecessor may have written has to be read
+wait (wait_previous, after_previous), and what the predecessor may have written has to be read
 with ordinary loads: neither __ldg nor a const __restrict__ parameter, which
 promise memory that nothing writes during the kernel's life.  The sources are
 checked here; on the GPU, chains of dependent calls without a host
@@ -63,7 +63,7 @@ def test_every_overlapped_kernel_waits():
         launched = set(re.findall(r"launch_overlapped\(\s*(\w+)<", text))
         assert launched
         for kernel in launched:
-            assert "after_previous()" in _function(source, kernel)[1], kernel
+            assert re.search(r"(after|wait)_previous\(\)", _function(source, kernel)[1]), kernel
             assert kernel in WRITTEN[source], kernel
 
 
