@@ -467,7 +467,8 @@ def union_systems(systems):
 
 class Batch:
     """Independent systems stored as consecutive row ranges of one union
-    pattern, solved together by batch_sqmr_solve (one CTA per system)."""
+    pattern, solved together by batch_sqmr_solve (one CTA per system, or the
+    whole grid where the largest system would hold the batch up)."""
 
     def __init__(self, pattern: Pattern, row_offsets):
         self.pattern = pattern

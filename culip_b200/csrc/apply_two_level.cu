@@ -9,11 +9,12 @@
 // Both load what belongs to the factor while the kernel before them drains
 // (launch.cuh).
 //
-// The arithmetic and its order are k_sweep_level's (solve.cu).  Bound: L1 tag
-// throughput and the tile's serial substitution.  With a lane per row every
-// load of a warp touches up to 32 lines; a tile's run of U' is therefore read
-// across the lanes (coalesced, gathers all in flight) into shared memory, where
-// each lane then sums its own row.  A division in the chain is taken only
+// The arithmetic and its order are k_sweep_level's (solve.cu).  Bound: dependent
+// loads and the tile's serial substitution (scale system, FP64: L1TEX at 36 to
+// 55 % of its peak, L2 and DRAM below 26 %).  With a lane per row every load of
+// a warp touches up to 32 lines; a tile's run of U' is therefore read across the
+// lanes (coalesced, gathers all in flight) into shared memory, where each lane
+// then sums its own row.  A division in the chain is taken only
 // where the tile's diagonal is not 1.  Measured, LEFT / RIGHT with k_sweep_level
 // against this: scale FP64 21.3 / 18.1 -> 13.6 / 12.6 us, N = 1.5 M FP32
 // 51 / 47 -> 38.5 / 39 us.

@@ -21,8 +21,9 @@
 // are dropped.  Zeros that the general path multiplies with a NaN or an
 // infinity are not in K's rows: spread_nonfinite puts their NaN in.
 //
-// Bound: the tiles' serial pivot steps (short scoreboard and fixed latency, an
-// issue slot in three used), not bandwidth.  Measured on the scale system
+// Bound: the tiles' serial pivot steps (dependent loads and fixed latency, an
+// issue slot in three used), not bandwidth; the order kernel's L1 requests
+// (L1TEX at 76 %).  Measured on the scale system
 // (n = 200 000, m = 100 000, 3125 tiles of 32, FP64): 120 us (rows 13, tiles
 // 85, order 22) against 960 us for the general path's 31 launches, 590 of them
 // in the tiles' block-by-block updates; N = 3000 with tiles of 4: 18 us against
